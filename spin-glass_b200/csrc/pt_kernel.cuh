@@ -115,14 +115,25 @@ __host__ __device__ constexpr int nseg_option(int L, int i) {
 }
 __host__ __device__ constexpr int threads_per_quad(int L, int nseg) { return L * (L / 2) * nseg; }
 
-__device__ __forceinline__ uint32_t maj3(uint32_t a, uint32_t b, uint32_t c) {
-    return (a & b) | (a & c) | (b & c);
+// One three-input logic instruction with truth table LUT (a = 0xF0, b = 0xCC,
+// c = 0xAA).  The update path is bound by the logic pipe (64 lanes per clock
+// and SM), so its gates are pinned one by one: left as C expressions, the
+// compiler reassociated the XORs across the adders and a site word took 49
+// logic instructions beside its Philox share instead of the 23 written (55 to
+// 29 with it at L = 16).
+template <int LUT>
+__device__ __forceinline__ uint32_t lop3(uint32_t a, uint32_t b, uint32_t c) {
+    uint32_t d;
+    asm("lop3.b32 %0, %1, %2, %3, %4;" : "=r"(d) : "r"(a), "r"(b), "r"(c), "n"(LUT));
+    return d;
 }
+__device__ __forceinline__ uint32_t xor3(uint32_t a, uint32_t b, uint32_t c) { return lop3<0x96>(a, b, c); }
+__device__ __forceinline__ uint32_t maj3(uint32_t a, uint32_t b, uint32_t c) { return lop3<0xE8>(a, b, c); }
 
 #define CSG_FA(s, cy, a, b, c)                             \
     do {                                                   \
         const uint32_t fa_a = (a), fa_b = (b), fa_c = (c); \
-        (s) = fa_a ^ fa_b ^ fa_c;                          \
+        (s) = xor3(fa_a, fa_b, fa_c);                      \
         (cy) = maj3(fa_a, fa_b, fa_c);                     \
     } while (0)
 
@@ -272,20 +283,42 @@ __device__ __forceinline__ void packed_column_counts(const uint32_t (&v)[4][NLV]
     }
 }
 
-// Flip mask at H = 0: U >= 3 always accepted; U = 2, 1, 0 accepted when the
-// draw is below thr[U] (t2, t1, t0; t0 <= t1 <= t2).
+// All ones where r < t, else zero: the borrow of r - t.  The subtraction runs
+// on the logic/add pipe and the borrow's spread on the multiply pipe; a
+// compare and a select (of any value) are two instructions of the former.
+// (A mask from one 64-bit multiply-add, r * 1 + (2^64 - t), leaves the logic
+// pipe out altogether, but its 64-bit addends cost dispatch slots and
+// registers: 5 to 9 % slower in the resident kernel at L = 12..20.)
+__device__ __forceinline__ uint32_t below(uint32_t r, uint32_t t) {
+    uint32_t m;
+    asm("{\n .reg .u32 d;\n sub.cc.u32 d, %1, %2;\n subc.u32 %0, 0, 0;\n}" : "=r"(m) : "r"(r), "r"(t));
+    return m;
+}
+
+// Flip at H = 0: U >= 3 always accepted; U = 2, 1, 0 accepted when the draw is
+// below t2, t1, t0 (t0 <= t1 <= t2).  With j the number of those thresholds
+// above the draw, a flip is accepted iff U + j >= 3; from the two full adders
+// (U = sa + sb + 2(ca + cb)) and the three masks that takes four gates and
+// the OR of the two terms, which the caller's own gate absorbs.  (Found by an
+// exhaustive search over gate pairs; three compares, five gates and three
+// selects did the same in eleven.)
+struct FlipTerms {
+    uint32_t x, y;  // flip = x | y
+};
+__device__ __forceinline__ FlipTerms flip_h0_terms(uint32_t sa, uint32_t ca, uint32_t sb, uint32_t cb,
+                                                   uint32_t r, uint32_t t0, uint32_t t1, uint32_t t2) {
+    const uint32_t m0 = below(r, t0), m1 = below(r, t1), m2 = below(r, t2);
+    const uint32_t g = lop3<0x61>(ca, cb, m0);
+    const uint32_t h = lop3<0x7E>(sa, m2, g);
+    return FlipTerms{lop3<0xE2>(ca, g, h), lop3<0xD4>(sb, m1, h)};
+}
 __device__ __forceinline__ uint32_t flip_h0(uint32_t sa, uint32_t ca, uint32_t sb, uint32_t cb,
                                             uint32_t r, uint32_t t0, uint32_t t1, uint32_t t2) {
-    const uint32_t v = sa | sb;
-    const uint32_t ge1 = ca | cb | v;
-    const uint32_t ge2 = ca | cb | (sa & sb);
-    const uint32_t ge3 = maj3(ca, cb, v);
-    uint32_t f = ge3;
-    f = (r < t2) ? ge2 : f;
-    f = (r < t1) ? ge1 : f;
-    f = (r < t0) ? 0xFFFFFFFFu : f;
-    return f;
+    const FlipTerms f = flip_h0_terms(sa, ca, sb, cb, r, t0, t1, t2);
+    return f.x | f.y;
 }
+// s ^ (x | y): the flipped spin word in one gate
+__device__ __forceinline__ uint32_t flipped(uint32_t s, const FlipTerms& f) { return lop3<0x1E>(s, f.x, f.y); }
 
 // General field, 0 <= H <= 4.  A flip of centre spin s with U unsatisfied
 // bonds is accepted iff U >= ucut_s (dE <= 0) or the draw r < thr[s][U].

@@ -61,26 +61,25 @@ __device__ __forceinline__ void add_plane_counts(const uint32_t (&v)[4][NLV], in
 }
 
 // Sites per thread up to which a colour pass is unrolled completely; longer
-// columns run as a loop over pairs of sites.
+// columns run as a loop over groups of sites.
 #ifndef CSG_UNROLL_ALL_ZS
 #define CSG_UNROLL_ALL_ZS 8
 #endif
 constexpr int kUnrollAllZS = CSG_UNROLL_ALL_ZS;
-// Longer columns run as a loop over groups of sites: the largest even divisor
-// of the column length up to this many.
-#ifndef CSG_SITE_GROUP
-#define CSG_SITE_GROUP 4
-#endif
-// 1: one copy of the colour pass serves both colours, the energy counting
-// guarded by a flag (half the code); 0: a copy with and one without counting.
-#ifndef CSG_RUNTIME_ACC
-#define CSG_RUNTIME_ACC 0
-#endif
-constexpr bool kRuntimeAcc = CSG_RUNTIME_ACC != 0;
+// Longer columns run as a loop over groups of sites, the largest even divisor
+// of the column length up to kSiteGroup.  A group's pointers are advanced once
+// (about 28 instructions of the logic/add pipe): at L = 16, Metropolis only, a
+// sweep takes 14.2 us with groups of 4 and 13.4 with 8.  The whole column
+// unrolled takes 12.9 alone but 27.6 instead of 24.5 us with an exchange and a
+// measurement every sweep (at L = 12: 16.5 instead of 12.3): copies of the
+// pass, ~750 bytes a site, then fall out of the instruction cache.  Groups
+// that do not tile the column, with a shorter tail, were slower too (L = 14,
+// 10 words: 7.4 against 6.5 us with groups of 2).
+constexpr int kSiteGroup = 10;
 
-__host__ __device__ constexpr int site_group(int zs, int cap) {
+__host__ __device__ constexpr int site_group(int zs) {
     int u = 2;
-    for (int d = 2; d <= cap && d <= zs; d += 2)
+    for (int d = 2; d <= kSiteGroup && d <= zs; d += 2)
         if (zs % d == 0) u = d;
     return u;
 }
@@ -218,10 +217,9 @@ __global__ void __launch_bounds__(max_cta_threads(GEN_H, NSEG)) pt_resident_kern
 #pragma unroll
             for (int l = 0; l < NLV; ++l) ecnt[k][l] = 0;
 
-        // one colour of the checkerboard; ACC (and, with runtime counting,
-        // accum): also add the post-flip unsatisfied-bond counts into the
-        // energy counters
-        auto colour_pass = [&](const int p, auto acc_tag, const bool accum) {
+        // one colour of the checkerboard; ACC: also add the post-flip
+        // unsatisfied-bond counts into the energy counters
+        auto colour_pass = [&](const int p, auto acc_tag) {
             constexpr bool ACC = decltype(acc_tag)::value;
             // x parity of the column's sites alternates along z: sites k = 0, 2, ...
             // have x = 2h + o0, sites k = 1, 3, ... x = 2h + 1 - o0
@@ -266,37 +264,36 @@ __global__ void __launch_bounds__(max_cta_threads(GEN_H, NSEG)) pt_resident_kern
 #pragma unroll
                 for (int kq = 0; kq < 4; ++kq) {
                     const uint32_t s0 = cw[kq];
-                    const uint32_t u0 = s0 ^ n0w[kq] ^ f0, u1 = s0 ^ n1w[kq] ^ f1;
-                    const uint32_t u2 = s0 ^ n2w[kq] ^ f2, u3 = s0 ^ n3w[kq] ^ f3;
-                    const uint32_t u4 = s0 ^ n4w[kq] ^ f4, u5 = s0 ^ n5w[kq] ^ f5;
-                    const uint32_t sa = u0 ^ u1 ^ u2, ca = maj3(u0, u1, u2);
-                    const uint32_t sb = u3 ^ u4 ^ u5, cb = maj3(u3, u4, u5);
+                    const uint32_t u0 = xor3(s0, n0w[kq], f0), u1 = xor3(s0, n1w[kq], f1);
+                    const uint32_t u2 = xor3(s0, n2w[kq], f2), u3 = xor3(s0, n3w[kq], f3);
+                    const uint32_t u4 = xor3(s0, n4w[kq], f4), u5 = xor3(s0, n5w[kq], f5);
+                    const uint32_t sa = xor3(u0, u1, u2), ca = maj3(u0, u1, u2);
+                    const uint32_t sb = xor3(u3, u4, u5), cb = maj3(u3, u4, u5);
                     uint32_t fl;
-                    if constexpr (GEN_H)
+                    if constexpr (GEN_H) {
                         fl = flip_gen(s0, sa, ca, sb, cb, rr[kq], thrq[2 * kq], thrq[2 * kq + 1],
                                       (int)((uc0 >> (8 * kq)) & 0xFF), (int)((uc1 >> (8 * kq)) & 0xFF));
-                    else
-                        fl = flip_h0(sa, ca, sb, cb, rr[kq], th0[kq], th1[kq], th2[kq]);
-                    cw[kq] = s0 ^ fl;
+                        cw[kq] = s0 ^ fl;
+                    } else {
+                        const FlipTerms ft = flip_h0_terms(sa, ca, sb, cb, rr[kq], th0[kq], th1[kq], th2[kq]);
+                        fl = ft.x | ft.y;
+                        cw[kq] = flipped(s0, ft);
+                    }
                     if constexpr (ACC) {
-                        if (accum) {
-                            wd[kq][0] = sa ^ fl;
-                            wd[kq][1] = sb ^ fl;
-                            wd[kq][2] = ca ^ fl;
-                            wd[kq][3] = cb ^ fl;
-                        }
+                        wd[kq][0] = sa ^ fl;
+                        wd[kq][1] = sb ^ fl;
+                        wd[kq][2] = ca ^ fl;
+                        wd[kq][3] = cb ^ fl;
                     }
                 }
                 st4(Sc, off, make_uint4(cw[0], cw[1], cw[2], cw[3]));
             };
             auto acc2 = [&](const uint32_t (&wa)[4][4], const uint32_t (&wb)[4][4]) {
                 if constexpr (ACC) {
-                    if (accum) {
 #pragma unroll
-                        for (int kq = 0; kq < 4; ++kq)
-                            vc_add_2sites<NLV>(ecnt[kq], wa[kq][0], wa[kq][1], wa[kq][2], wa[kq][3],
-                                               wb[kq][0], wb[kq][1], wb[kq][2], wb[kq][3]);
-                    }
+                    for (int kq = 0; kq < 4; ++kq)
+                        vc_add_2sites<NLV>(ecnt[kq], wa[kq][0], wa[kq][1], wa[kq][2], wa[kq][3],
+                                           wb[kq][0], wb[kq][1], wb[kq][2], wb[kq][3]);
                 }
             };
             if constexpr (ZS <= kUnrollAllZS) {
@@ -308,18 +305,16 @@ __global__ void __launch_bounds__(max_cta_threads(GEN_H, NSEG)) pt_resident_kern
                         site(k + 1, true, -PL, k + 1 == ZS - 1 ? dzL : PL, wb);
                         acc2(wa, wb);
                     } else if constexpr (ACC) {
-                        if (accum) {
 #pragma unroll
-                            for (int kq = 0; kq < 4; ++kq)
-                                vc_add_site<NLV>(ecnt[kq], wa[kq][0], wa[kq][1], wa[kq][2], wa[kq][3]);
-                        }
+                        for (int kq = 0; kq < 4; ++kq)
+                            vc_add_site<NLV>(ecnt[kq], wa[kq][0], wa[kq][1], wa[kq][2], wa[kq][3]);
                     }
                 }
             } else {
-                // groups of U sites: a group's sites sit at fixed offsets from
-                // its first one; only the first group's first site and the last
-                // group's last site wrap around in z
-                constexpr int U = site_group(ZS, CSG_SITE_GROUP);
+                // a group's sites sit at fixed offsets from its first one; only
+                // the first group's first site and the last group's last site
+                // wrap around in z
+                constexpr int U = site_group(ZS);
                 static_assert(ZS % U == 0 && U % 2 == 0, "groups must tile the column");
 #pragma unroll 1
                 for (int k0 = 0; k0 < ZS; k0 += U) {
@@ -335,19 +330,13 @@ __global__ void __launch_bounds__(max_cta_threads(GEN_H, NSEG)) pt_resident_kern
                 }
             }
         };
-        if constexpr (kRuntimeAcc) {
-            if (active) colour_pass(0, std::true_type{}, false);
-            __syncthreads();
-            if (active) colour_pass(1, std::true_type{}, need_E);
-        } else {
-            if (active) colour_pass(0, std::false_type{}, false);
-            __syncthreads();
-            if (active) {
-                if (need_E)
-                    colour_pass(1, std::true_type{}, true);
-                else
-                    colour_pass(1, std::false_type{}, false);
-            }
+        if (active) colour_pass(0, std::false_type{});
+        __syncthreads();
+        if (active) {
+            if (need_E)
+                colour_pass(1, std::true_type{});
+            else
+                colour_pass(1, std::false_type{});
         }
         __syncthreads();
 

@@ -99,21 +99,23 @@ __global__ void __launch_bounds__(colour_threads<ACC_E || ACC_M>()) stream_colou
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
             const uint32_t s0 = cw[k];
-            const uint32_t u0 = s0 ^ n0w[k] ^ f0, u1 = s0 ^ n1w[k] ^ f1;
-            const uint32_t u2 = s0 ^ n2w[k] ^ f2, u3 = s0 ^ n3w[k] ^ f3;
-            const uint32_t u4 = s0 ^ n4w[k] ^ f4, u5 = s0 ^ n5w[k] ^ f5;
-            const uint32_t sa = u0 ^ u1 ^ u2, ca = maj3(u0, u1, u2);
-            const uint32_t sb = u3 ^ u4 ^ u5, cb = maj3(u3, u4, u5);
+            const uint32_t u0 = xor3(s0, n0w[k], f0), u1 = xor3(s0, n1w[k], f1);
+            const uint32_t u2 = xor3(s0, n2w[k], f2), u3 = xor3(s0, n3w[k], f3);
+            const uint32_t u4 = xor3(s0, n4w[k], f4), u5 = xor3(s0, n5w[k], f5);
+            const uint32_t sa = xor3(u0, u1, u2), ca = maj3(u0, u1, u2);
+            const uint32_t sb = xor3(u3, u4, u5), cb = maj3(u3, u4, u5);
             uint32_t fl;
             if constexpr (GEN_H) {
                 uint4 ta, tb;
                 gen_thresholds(P.tab, 4 * q + k, ta, tb);
                 fl = flip_gen(s0, sa, ca, sb, cb, rr[k], ta, tb, P.tab.ucut[4 * q + k][0],
                               P.tab.ucut[4 * q + k][1]);
+                cw[k] = s0 ^ fl;
             } else {
-                fl = flip_h0(sa, ca, sb, cb, rr[k], th0[k], th1[k], th2[k]);
+                const FlipTerms ft = flip_h0_terms(sa, ca, sb, cb, rr[k], th0[k], th1[k], th2[k]);
+                fl = ft.x | ft.y;
+                cw[k] = flipped(s0, ft);
             }
-            cw[k] = s0 ^ fl;
             // post-flip unsatisfied bonds (energy) and spins up, counted at once
             if constexpr (ACC_E) {
                 wd[k][0] = sa ^ fl;

@@ -248,18 +248,21 @@ __global__ void __launch_bounds__(kSweepMaxThreads) stream_sweep_kernel(const __
 #pragma unroll
         for (int kq = 0; kq < 4; ++kq) {
             const uint32_t s0 = cw[kq];
-            const uint32_t u0 = s0 ^ n0w[kq] ^ f0, u1 = s0 ^ n1w[kq] ^ f1;
-            const uint32_t u2 = s0 ^ n2w[kq] ^ f2, u3 = s0 ^ n3w[kq] ^ f3;
-            const uint32_t u4 = s0 ^ n4w[kq] ^ f4, u5 = s0 ^ n5w[kq] ^ f5;
-            const uint32_t sa = u0 ^ u1 ^ u2, ca = maj3(u0, u1, u2);
-            const uint32_t sb = u3 ^ u4 ^ u5, cb = maj3(u3, u4, u5);
+            const uint32_t u0 = xor3(s0, n0w[kq], f0), u1 = xor3(s0, n1w[kq], f1);
+            const uint32_t u2 = xor3(s0, n2w[kq], f2), u3 = xor3(s0, n3w[kq], f3);
+            const uint32_t u4 = xor3(s0, n4w[kq], f4), u5 = xor3(s0, n5w[kq], f5);
+            const uint32_t sa = xor3(u0, u1, u2), ca = maj3(u0, u1, u2);
+            const uint32_t sb = xor3(u3, u4, u5), cb = maj3(u3, u4, u5);
             uint32_t fl;
-            if constexpr (GEN_H)
+            if constexpr (GEN_H) {
                 fl = flip_gen(s0, sa, ca, sb, cb, rr[kq], sThr[kq][0], sThr[kq][1],
                               P.tab.ucut[4 * q + kq][0], P.tab.ucut[4 * q + kq][1]);
-            else
-                fl = flip_h0(sa, ca, sb, cb, rr[kq], th0[kq], th1[kq], th2[kq]);
-            cw[kq] = s0 ^ fl;
+                cw[kq] = s0 ^ fl;
+            } else {
+                const FlipTerms ft = flip_h0_terms(sa, ca, sb, cb, rr[kq], th0[kq], th1[kq], th2[kq]);
+                fl = ft.x | ft.y;
+                cw[kq] = flipped(s0, ft);
+            }
             wd[kq][0] = sa ^ fl;
             wd[kq][1] = sb ^ fl;
             wd[kq][2] = ca ^ fl;
