@@ -314,18 +314,15 @@ constexpr int64_t kSweepsPerLaunch = 1024;
 // sequence of one sweep.
 // ---------------------------------------------------------------------------
 struct StreamLayout {
-    int nblk = 0, nblk_plain = 0, nblk2 = 0;
+    int nblk2 = 0;
     size_t u_acc = 0, up_acc = 0, d_acc = 0, energy = 0, magn = 0, masks = 0, err = 0, bytes = 0;
 };
 
 StreamLayout stream_layout(const csg_config& c) {
     const csg_dims& d = c.dims;
     const size_t N = (size_t)d.L * d.L * d.L;
-    const size_t spb = (size_t)csg::kStreamThreads * csg::kStreamSPT;
-    const size_t spa = csg::kStreamAccSitesPerBlock, spo = csg::kOverlapSitesPerBlock;
+    const size_t spo = csg::kOverlapSitesPerBlock;
     StreamLayout s;
-    s.nblk = (int)((N / 2 + spa - 1) / spa);  // blocks of the counting colour launches
-    s.nblk_plain = (int)((N / 2 + spb - 1) / spb);
     s.nblk2 = (int)((N + spo - 1) / spo);
     const size_t planes = (size_t)d.n_words * d.n_copies * d.n_temps;
     auto up = [](size_t b) { return (b + 255) & ~(size_t)255; };
@@ -359,23 +356,50 @@ cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, cudaStre
     return cudaLaunchKernelEx(&lc, kernel, std::forward<Args>(args)...);
 }
 
-using ColourLaunch = void (*)(const csg::StreamParams&, const StreamLayout&, int, long long,
-                              cudaStream_t);
-
-template <bool G, bool E, bool M>
-void launch_colour(const csg::StreamParams& S, const StreamLayout& lay, int p, long long s,
-                   cudaStream_t st) {
-    const dim3 grid((unsigned)(S.W * S.C * S.Q), (unsigned)(E || M ? lay.nblk : lay.nblk_plain));
-    launch_pdl(csg::stream_colour_kernel<G, E, M>, grid, dim3(csg::colour_threads<E || M>()), st, S, p, s);
+// Planes per block of a colour launch: the cheapest in waves of resident blocks
+// times a block's time, counted in planes plus what a block costs besides (its
+// set-up, about one; counting launches also reduce their counters, about four).
+int colour_planes(const csg::StreamParams& S, int copies, int blocks_per_sm, int nsm, bool counting) {
+    const int extra = counting ? 4 : 1;
+    const long per_chunk = (long)S.W * (S.C / copies) * S.Q *
+                           ((S.L * (S.L / 2) + csg::kColourThreads - 1) / csg::kColourThreads);
+    const long slots = (long)blocks_per_sm * nsm;
+    int best = 2;
+    long best_cost = -1;
+    for (int zb = 2; zb <= csg::kColourMaxZ && zb <= S.L; zb += 2) {
+        const long blocks = per_chunk * ((S.L + zb - 1) / zb);
+        const long cost = (blocks + slots - 1) / slots * (zb + extra);
+        if (best_cost < 0 || cost <= best_cost) {
+            best_cost = cost;
+            best = zb;
+        }
+    }
+    return best;
 }
 
-ColourLaunch colour_launch(bool gen, bool acc_e, bool acc_m) {
+using ColourLaunch = void (*)(const csg::StreamParams&, int, int, long long, cudaStream_t);
+
+template <bool G, bool E, bool M, int C>
+void launch_colour(const csg::StreamParams& S, int nsm, int p, long long s, cudaStream_t st) {
+    constexpr int NC = csg::colour_copies<E || M>(C);
+    const int zb = colour_planes(S, NC, csg::colour_blocks<G, E, M, NC>(), nsm, E || M);
+    const int npb = (S.L * (S.L / 2) + csg::kColourThreads - 1) / csg::kColourThreads;
+    const dim3 grid((unsigned)(S.W * (S.C / NC) * S.Q), (unsigned)(npb * ((S.L + zb - 1) / zb)));
+    launch_pdl(csg::stream_colour_kernel<G, E, M, NC>, grid, dim3(csg::kColourThreads), st, S, p, s, zb);
+}
+
+template <int C>
+ColourLaunch colour_launch_of(bool gen, bool acc_e, bool acc_m) {
     static const ColourLaunch fns[8] = {
-        launch_colour<false, false, false>, launch_colour<false, false, true>,
-        launch_colour<false, true, false>,  launch_colour<false, true, true>,
-        launch_colour<true, false, false>,  launch_colour<true, false, true>,
-        launch_colour<true, true, false>,   launch_colour<true, true, true>};
+        launch_colour<false, false, false, C>, launch_colour<false, false, true, C>,
+        launch_colour<false, true, false, C>,  launch_colour<false, true, true, C>,
+        launch_colour<true, false, false, C>,  launch_colour<true, false, true, C>,
+        launch_colour<true, true, false, C>,   launch_colour<true, true, true, C>};
     return fns[(gen ? 4 : 0) + (acc_e ? 2 : 0) + (acc_m ? 1 : 0)];
+}
+
+ColourLaunch colour_launch(int copies, bool gen, bool acc_e, bool acc_m) {
+    return copies == 2 ? colour_launch_of<2>(gen, acc_e, acc_m) : colour_launch_of<1>(gen, acc_e, acc_m);
 }
 
 // Same schedule, Philox counters and arithmetic as the resident kernel's sweep
@@ -397,15 +421,11 @@ int run_stream(const csg_config& cfg, uint32_t* spins, const uint32_t* bonds,
     S.C = d.n_copies;
     S.T = d.n_temps;
     S.Q = d.n_temps / 4;
-    S.nblk = lay.nblk;
     S.nblk2 = lay.nblk2;
     S.k0 = tp.k0;
     S.k1 = tp.k1;
     S.word0 = tp.word0;
     S.H = tp.H;
-    auto magic = [](uint64_t d) { return (uint32_t)(((uint64_t)1 << 32) / d + ((((uint64_t)1 << 32) % d) ? 1 : 0)); };
-    S.mag_plane = magic((uint64_t)d.L * (d.L / 2));
-    S.mag_row = magic((uint64_t)(d.L / 2));
     S.tab = tp.tab;
     csg::StreamObs O{};
     unsigned long long *boundary = nullptr, *swap_acc = nullptr;
@@ -427,6 +447,9 @@ int run_stream(const csg_config& cfg, uint32_t* spins, const uint32_t* bonds,
         log_rounds = obs->swap_log_rounds;
         round0 = obs->swap_round0;
     }
+    int dev = 0, nsm = 0;
+    CSG_CUDA(cudaGetDevice(&dev));
+    CSG_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
     char* base = nullptr;
     CSG_CUDA(cudaMallocAsync(reinterpret_cast<void**>(&base), lay.bytes, st));
     S.u_acc = reinterpret_cast<int*>(base + lay.u_acc);
@@ -458,8 +481,8 @@ int run_stream(const csg_config& cfg, uint32_t* spins, const uint32_t* bonds,
             ce = csg::launch_stream_sweep(S, s, gen, need_E, need_M, st);
             if (ce != cudaSuccess) break;
         } else {
-            colour_launch(gen, false, need_M)(S, lay, 0, s, st);
-            colour_launch(gen, need_E, need_M)(S, lay, 1, s, st);
+            colour_launch(d.n_copies, gen, false, need_M)(S, nsm, 0, s, st);
+            colour_launch(d.n_copies, gen, need_E, need_M)(S, nsm, 1, s, st);
         }
         if (need_E) {
             const long long round = do_swap ? (s + 1) / sps - 1 : 0;

@@ -22,172 +22,223 @@
 
 namespace csg {
 
-// One colour of one sweep.  blockIdx.x = quad (w, c, q), blockIdx.y = block
-// of colour_spt * blockDim.x sites of that colour; each thread updates
-// colour_spt sites in the 4 planes of the quad.  Consecutive blocks take the
-// quads of one word at the same sites, so the word's bonds are read once from
-// DRAM and then from L2.
-template <bool GEN_H, bool ACC_E, bool ACC_M>
-__global__ void __launch_bounds__(colour_threads<ACC_E || ACC_M>()) stream_colour_kernel(
-    const __grid_constant__ StreamParams P, int p, long long s) {
+// Address of element off of an array of 4- or 16-byte elements: one multiply-add
+// on the multiply pipe.  Left to itself the compiler keeps a 64-bit pointer per
+// neighbour and advances each with two adds on the logic/add pipe, which bounds
+// the update.
+template <typename T>
+__device__ __forceinline__ T* elem(T* base, uint32_t off) {
+    uint64_t a;
+    asm("mad.wide.u32 %0, %1, %2, %3;" : "=l"(a) : "r"(off), "n"(sizeof(T)), "l"(base));
+    return reinterpret_cast<T*>(a);
+}
+
+__device__ __forceinline__ void prefetch_l1(const void* a) {
+    asm volatile("prefetch.global.L1 [%0];" ::"l"(a));
+}
+
+// One colour of one sweep.  blockIdx.x = (w, q) for NC = 2 copies at once,
+// (w, c, q) for NC = 1; blockIdx.y = block of kColourThreads sites of a
+// z-plane x chunk of zb z-planes: a thread takes one site (y, h) of the
+// plane's half in NC quads and walks zb planes along z, so that its in-plane
+// neighbour offsets are fixed for the launch and the other colour's words at
+// z - 1 and z are carried from plane to plane (5 instead of 7 loads of 16
+// bytes a site).  The two copies of a temperature quad share its bonds,
+// thresholds and addresses.  Consecutive blocks take the quads of one word at
+// the same sites, so the word's bonds are read once from DRAM and then from L2.
+// Bound: logic pipe and issue (56 and 60 % busy) with the latency of the loads
+// that miss L1 in between.  256 samples, 2 copies, 32 temperatures, a launch:
+// L = 48, 97 -> 75 us (counting: 133 -> 115); L = 32, 29 -> 25 (47 -> 37)
+// against a thread per site with 7 loads and index arithmetic for each.
+template <bool GEN_H, bool ACC_E, bool ACC_M, int NC>
+__global__ void __launch_bounds__(kColourThreads, colour_blocks<GEN_H, ACC_E, ACC_M, NC>())
+    stream_colour_kernel(const __grid_constant__ StreamParams P, int p, long long s, int zb) {
     pdl_enter();
-    const int L = P.L, LH = L / 2;
-    const int N = L * L * L, NH = N / 2;
-    const int gq = blockIdx.x;
-    const int w = gq / (P.C * P.Q), c = (gq / P.Q) % P.C, q = gq % P.Q;
-    uint4* Sq = reinterpret_cast<uint4*>(P.spins) + (size_t)gq * N;
-    uint4* Sc = Sq + p * NH;
-    const uint4* So = Sq + (1 - p) * NH;
-    const uint32_t* Fw = P.bonds + (size_t)w * 3 * N;
-    const uint32_t* Fc = Fw + p * NH;
-    const uint32_t* Fo = Fw + (1 - p) * NH;
-    const uint32_t ctr3 = kTagSweep | ((uint32_t)c << 8) | (uint32_t)q;
-    const uint32_t wg = (uint32_t)w + P.word0;
-    // the Philox rounds that do not depend on the site, once per launch
-    const PhiloxFixed pf = philox_fix((uint32_t)s, wg, ctr3, P.k0, P.k1);
+    constexpr int NLV = kStreamNLV, NLM = kStreamNLM;
+    const int L = P.L, LH = L / 2, PL = L * LH;
+    const int N = L * PL * 2, NH = L * PL;
+    // quad gq0 + c * Q, c = 0 .. NC - 1
+    const int bx = blockIdx.x, Q = P.Q;
+    const int w = NC == 1 ? bx / (P.C * Q) : bx / Q, q = bx % Q;
+    const int c0 = NC == 1 ? (bx / Q) % P.C : 0;
+    const size_t gq0 = (size_t)(w * P.C + c0) * Q + q;
+    const int npb = (PL + kColourThreads - 1) / kColourThreads;
+    const int zc = blockIdx.y / npb, pb = blockIdx.y - zc * npb;
+    const int z0 = zc * zb, z1 = min(L, z0 + zb);
     const int lane = threadIdx.x & 31;
-    uint32_t th0[4], th1[4], th2[4];
+    const int i = pb * kColourThreads + threadIdx.x;  // (y, h) of the plane's half
+    const bool active = i < PL;
+
+    uint32_t ecnt[NC][4][NLV], mcnt[NC][4][NLM];
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-        const int t = 4 * q + k;
-        th0[k] = P.tab.thr[t][0][0];
-        th1[k] = P.tab.thr[t][0][1];
-        th2[k] = P.tab.thr[t][0][2];
-    }
-    constexpr int NLV = kStreamNLV;
-    constexpr int NLM = kStreamNLM;
-    // Bit-sliced counters of the counting launches, one column per thread in
-    // shared memory (conflict-free): held in registers they cost ~30 registers
-    // per thread and with them resident blocks (measured 5 % slower at L=48).
-    constexpr int BTS = colour_threads<ACC_E || ACC_M>();
-    __shared__ uint32_t s_cnt[(ACC_E ? 4 * NLV : 0) + (ACC_M ? 4 * NLM : 0) + 1][BTS];
-    uint32_t* ecb = &s_cnt[0][threadIdx.x];                        // [4][NLV], stride BTS
-    uint32_t* mcb = &s_cnt[ACC_E ? 4 * NLV : 0][threadIdx.x];      // [4][NLM], stride BTS
-    if constexpr (ACC_E || ACC_M) {
-        for (int i = 0; i < (ACC_E ? 4 * NLV : 0) + (ACC_M ? 4 * NLM : 0); ++i) ecb[i * BTS] = 0;
-    }
-    const int PL = L * LH;  // sites of one colour in one z plane
-    constexpr int BT = colour_threads<ACC_E || ACC_M>(), SPT = colour_spt<ACC_E || ACC_M>();
-    const int n_base = blockIdx.y * (BT * SPT) + threadIdx.x;
-    auto update_site = [&](const int n, uint32_t (&wd)[4][4]) {
-        if (n >= (int)NH) return;
-        // n = (z L + y) L/2 + h; divisions by multiply-high
-        const int z = div_magic(n, PL, P.mag_plane);
-        const int rem = n - z * PL;
-        const int y = div_magic(rem, LH, P.mag_row);
-        const int h = rem - y * LH;
-        const int o = (y + z + p) & 1;
-        const int x = 2 * h + o;
-        const int nxm = o ? n : (h == 0 ? n + LH - 1 : n - 1);
-        const int nxp = o ? (h == LH - 1 ? n - h : n + 1) : n;
-        const int nym = y == 0 ? n + PL - LH : n - LH;
-        const int nyp = y == L - 1 ? n - PL + LH : n + LH;
-        const int nzm = z == 0 ? n + (int)NH - PL : n - PL;
-        const int nzp = z == L - 1 ? n - (int)NH + PL : n + PL;
-        const uint4 cv = Sc[n];
-        const uint4 a0 = __ldg(So + nxm), a1 = __ldg(So + nxp), a2 = __ldg(So + nym),
-                    a3 = __ldg(So + nyp), a4 = __ldg(So + nzm), a5 = __ldg(So + nzp);
-        const uint32_t f0 = __ldg(Fo + nxm), f1 = __ldg(Fc + n);
-        const uint32_t f2 = __ldg(Fo + N + nym), f3 = __ldg(Fc + N + n);
-        const uint32_t f4 = __ldg(Fo + 2 * N + nzm), f5 = __ldg(Fc + 2 * N + n);
-        const u32x4 r = philox_c0((uint32_t)((z * L + y) * L + x), pf);
-        const uint32_t rr[4] = {r.v0, r.v1, r.v2, r.v3};
-        uint32_t cw[4] = {cv.x, cv.y, cv.z, cv.w};
-        const uint32_t n0w[4] = {a0.x, a0.y, a0.z, a0.w}, n1w[4] = {a1.x, a1.y, a1.z, a1.w};
-        const uint32_t n2w[4] = {a2.x, a2.y, a2.z, a2.w}, n3w[4] = {a3.x, a3.y, a3.z, a3.w};
-        const uint32_t n4w[4] = {a4.x, a4.y, a4.z, a4.w}, n5w[4] = {a5.x, a5.y, a5.z, a5.w};
+    for (int c = 0; c < NC; ++c)
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
-            const uint32_t s0 = cw[k];
-            const uint32_t u0 = xor3(s0, n0w[k], f0), u1 = xor3(s0, n1w[k], f1);
-            const uint32_t u2 = xor3(s0, n2w[k], f2), u3 = xor3(s0, n3w[k], f3);
-            const uint32_t u4 = xor3(s0, n4w[k], f4), u5 = xor3(s0, n5w[k], f5);
-            const uint32_t sa = xor3(u0, u1, u2), ca = maj3(u0, u1, u2);
-            const uint32_t sb = xor3(u3, u4, u5), cb = maj3(u3, u4, u5);
-            uint32_t fl;
-            if constexpr (GEN_H) {
-                uint4 ta, tb;
-                gen_thresholds(P.tab, 4 * q + k, ta, tb);
-                fl = flip_gen(s0, sa, ca, sb, cb, rr[k], ta, tb, P.tab.ucut[4 * q + k][0],
-                              P.tab.ucut[4 * q + k][1]);
-                cw[k] = s0 ^ fl;
-            } else {
-                const FlipTerms ft = flip_h0_terms(sa, ca, sb, cb, rr[k], th0[k], th1[k], th2[k]);
-                fl = ft.x | ft.y;
-                cw[k] = flipped(s0, ft);
+#pragma unroll
+            for (int l = 0; l < NLV; ++l) ecnt[c][k][l] = 0;
+#pragma unroll
+            for (int l = 0; l < NLM; ++l) mcnt[c][k][l] = 0;
+        }
+    if (active) {
+        const int y = i / LH, h = i - y * LH;
+        uint4* const Sq = reinterpret_cast<uint4*>(P.spins) + gq0 * N;
+        const size_t copy = (size_t)Q * N;  // from a quad to the other copy's
+        const uint32_t* const Fw = P.bonds + (size_t)w * 3 * N;
+        uint32_t th0[4], th1[4], th2[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const int t = 4 * q + k;
+            th0[k] = P.tab.thr[t][0][0];
+            th1[k] = P.tab.thr[t][0][1];
+            th2[k] = P.tab.thr[t][0][2];
+        }
+        // the Philox rounds that do not depend on the site, once per launch
+        PhiloxFixed pf[NC];
+#pragma unroll
+        for (int c = 0; c < NC; ++c)
+            pf[c] = philox_fix((uint32_t)s, (uint32_t)w + P.word0, kTagSweep | ((uint32_t)(c0 + c) << 8) | (uint32_t)q,
+                               P.k0, P.k1);
+        // x & 1 of the site in planes z0, z0 + 2, ... is o0, in the others 1 - o0.
+        // One x neighbour is the other colour's word at the same h (x + 1 of an
+        // even x, x - 1 of an odd one), the other one at h - 1 or h + 1.
+        const int o0 = (y + z0 + p) & 1;
+        // element offsets from plane z of colour 0; oc, oo: this colour's and
+        // the other's half
+        const uint32_t oc = (uint32_t)(p * NH + i), oo = (uint32_t)((1 - p) * NH + i);
+        const uint32_t iA = h == 0 ? oo + LH - 1 : oo - 1;     // x - 1 of an even x
+        const uint32_t iB = h == LH - 1 ? oo - h : oo + 1;     // x + 1 of an odd x
+        const uint32_t iE = o0 ? iB : iA, iO = o0 ? iA : iB;
+        const uint32_t iYm = y == 0 ? oo + PL - LH : oo - LH;
+        const uint32_t iYp = y == L - 1 ? oo - PL + LH : oo + LH;
+        // bonds of the x neighbours: at the same h, and at h -+ 1 (the bond to
+        // x - 1 belongs to the other colour's site, the one to x + 1 to this)
+        const uint32_t fsE = o0 ? oo : oc, fdE = o0 ? oc : iA, fsO = o0 ? oc : oo, fdO = o0 ? iA : oc;
+        const uint32_t f2o = (uint32_t)N + iYm, f3o = (uint32_t)N + oc;
+        const uint32_t f4o = 2u * N + oo, f5o = 2u * N + oc;
+        const uint32_t siteE = (uint32_t)(y * L + 2 * h + o0), siteO = (uint32_t)(y * L + 2 * h + 1 - o0);
+
+        uint4 zm[NC], zcur[NC];
+#pragma unroll
+        for (int c = 0; c < NC; ++c) {
+            zm[c] = *elem(Sq + c * copy + (size_t)(z0 == 0 ? L - 1 : z0 - 1) * PL, oo);
+            zcur[c] = *elem(Sq + c * copy + (size_t)z0 * PL, oo);
+        }
+        auto update_site = [&](const int z, const bool odd, uint32_t (&wd)[NC][4][4]) {
+            // the lines of the next two planes that no earlier load of this
+            // block brought in: on their way while this site is updated
+            // (L = 48: 75.0 us a launch instead of 79.5)
+            const int zn = z == L - 1 ? 0 : z + 1, zq = z >= L - 2 ? z + 2 - L : z + 2;
+#pragma unroll
+            for (int c = 0; c < NC; ++c) {
+                prefetch_l1(elem(Sq + c * copy + (size_t)zn * PL, oc));
+                prefetch_l1(elem(Sq + c * copy + (size_t)zq * PL, oo));
             }
-            // post-flip unsatisfied bonds (energy) and spins up, counted at once
+            const uint32_t* const F = Fw + (size_t)z * PL;
+            const uint32_t* const Fm = Fw + (size_t)(z == 0 ? L - 1 : z - 1) * PL;
+            const uint32_t f0 = __ldg(elem(F, odd ? fsO : fsE)), f1 = __ldg(elem(F, odd ? fdO : fdE));
+            const uint32_t f2 = __ldg(elem(F, f2o)), f3 = __ldg(elem(F, f3o));
+            const uint32_t f4 = __ldg(elem(Fm, f4o)), f5 = __ldg(elem(F, f5o));
+#pragma unroll
+            for (int c = 0; c < NC; ++c) {
+                uint4* const S = Sq + c * copy + (size_t)z * PL;
+                uint4* const Sp = Sq + c * copy + (size_t)zn * PL;
+                uint4* const own = elem(S, oc);
+                const uint4 cv = *own;
+                const uint4 an = *elem(Sp, oo);
+                const uint4 ad = *elem(S, odd ? iO : iE);
+                const uint4 a2 = *elem(S, iYm), a3 = *elem(S, iYp);
+                const u32x4 r = philox_c0((uint32_t)(z * L * L) + (odd ? siteO : siteE), pf[c]);
+                const uint32_t rr[4] = {r.v0, r.v1, r.v2, r.v3};
+                uint32_t cw[4] = {cv.x, cv.y, cv.z, cv.w};
+                const uint32_t n0w[4] = {zcur[c].x, zcur[c].y, zcur[c].z, zcur[c].w};
+                const uint32_t n1w[4] = {ad.x, ad.y, ad.z, ad.w};
+                const uint32_t n2w[4] = {a2.x, a2.y, a2.z, a2.w}, n3w[4] = {a3.x, a3.y, a3.z, a3.w};
+                const uint32_t n4w[4] = {zm[c].x, zm[c].y, zm[c].z, zm[c].w}, n5w[4] = {an.x, an.y, an.z, an.w};
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    const uint32_t s0 = cw[k];
+                    const uint32_t u0 = xor3(s0, n0w[k], f0), u1 = xor3(s0, n1w[k], f1);
+                    const uint32_t u2 = xor3(s0, n2w[k], f2), u3 = xor3(s0, n3w[k], f3);
+                    const uint32_t u4 = xor3(s0, n4w[k], f4), u5 = xor3(s0, n5w[k], f5);
+                    const uint32_t sa = xor3(u0, u1, u2), ca = maj3(u0, u1, u2);
+                    const uint32_t sb = xor3(u3, u4, u5), cb = maj3(u3, u4, u5);
+                    uint32_t fl;
+                    if constexpr (GEN_H) {
+                        uint4 ta, tb;
+                        gen_thresholds(P.tab, 4 * q + k, ta, tb);
+                        fl = flip_gen(s0, sa, ca, sb, cb, rr[k], ta, tb, P.tab.ucut[4 * q + k][0],
+                                      P.tab.ucut[4 * q + k][1]);
+                        cw[k] = s0 ^ fl;
+                    } else {
+                        const FlipTerms ft = flip_h0_terms(sa, ca, sb, cb, rr[k], th0[k], th1[k], th2[k]);
+                        fl = ft.x | ft.y;
+                        cw[k] = flipped(s0, ft);
+                    }
+                    // post-flip unsatisfied bonds (energy) and spins up, counted at once
+                    if constexpr (ACC_E) {
+                        wd[c][k][0] = sa ^ fl;
+                        wd[c][k][1] = sb ^ fl;
+                        wd[c][k][2] = ca ^ fl;
+                        wd[c][k][3] = cb ^ fl;
+                    }
+                    if constexpr (ACC_M) {
+                        uint32_t carry = cw[k];
+#pragma unroll
+                        for (int l = 0; l < NLM; ++l) {
+                            const uint32_t m = mcnt[c][k][l];
+                            mcnt[c][k][l] = m ^ carry;
+                            carry &= m;
+                        }
+                    }
+                }
+                *own = make_uint4(cw[0], cw[1], cw[2], cw[3]);
+                zm[c] = zcur[c];
+                zcur[c] = an;
+            }
+        };
+#pragma unroll 1
+        for (int z = z0; z < z1; z += 2) {  // L and zb are even
+            uint32_t wa[NC][4][4], wb[NC][4][4];
+            update_site(z, false, wa);
+            update_site(z + 1, true, wb);
             if constexpr (ACC_E) {
-                wd[k][0] = sa ^ fl;
-                wd[k][1] = sb ^ fl;
-                wd[k][2] = ca ^ fl;
-                wd[k][3] = cb ^ fl;
+#pragma unroll
+                for (int c = 0; c < NC; ++c)
+#pragma unroll
+                    for (int k = 0; k < 4; ++k)
+                        vc_add_2sites<NLV>(ecnt[c][k], wa[c][k][0], wa[c][k][1], wa[c][k][2], wa[c][k][3],
+                                           wb[c][k][0], wb[c][k][1], wb[c][k][2], wb[c][k][3]);
+            }
+        }
+    }
+    if constexpr (ACC_E || ACC_M) {
+        __shared__ int sred[NC][2][4][32];
+        for (int j = threadIdx.x; j < NC * 2 * 4 * 32; j += kColourThreads) (&sred[0][0][0][0])[j] = 0;
+        __syncthreads();
+#pragma unroll
+        for (int c = 0; c < NC; ++c) {
+            // all lanes of a block hold counters of its quad: the 4 planes of
+            // a warp in one 32x32 transpose per counter level
+            int cnt[4];
+            if constexpr (ACC_E) {
+                packed_column_counts<NLV>(ecnt[c], lane, cnt);
+#pragma unroll
+                for (int k = 0; k < 4; ++k) atomicAdd(&sred[c][0][k][lane], cnt[k]);
             }
             if constexpr (ACC_M) {
-                uint32_t carry = cw[k];
+                packed_column_counts<NLM>(mcnt[c], lane, cnt);
 #pragma unroll
-                for (int l = 0; l < NLM; ++l) {
-                    const uint32_t m = mcb[(k * NLM + l) * BTS];
-                    mcb[(k * NLM + l) * BTS] = m ^ carry;
-                    carry &= m;
-                }
+                for (int k = 0; k < 4; ++k) atomicAdd(&sred[c][1][k][lane], cnt[k]);
             }
         }
-        Sc[n] = make_uint4(cw[0], cw[1], cw[2], cw[3]);
-    };
-    // sites in pairs: the energy counters take both at once (fewer counter
-    // updates); the two updates themselves run one after the other
-    static_assert(SPT % 2 == 0, "sites are counted in pairs");
-#pragma unroll 1
-    for (int m = 0; m < SPT; m += 2) {
-        uint32_t wa[4][4] = {}, wb[4][4] = {};
-        update_site(n_base + m * BT, wa);
-        update_site(n_base + (m + 1) * BT, wb);
-        if constexpr (ACC_E) {
-#pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                uint32_t v[NLV];
-#pragma unroll
-                for (int l = 0; l < NLV; ++l) v[l] = ecb[(k * NLV + l) * BTS];
-                vc_add_2sites<NLV>(v, wa[k][0], wa[k][1], wa[k][2], wa[k][3], wb[k][0], wb[k][1],
-                                   wb[k][2], wb[k][3]);
-#pragma unroll
-                for (int l = 0; l < NLV; ++l) ecb[(k * NLV + l) * BTS] = v[l];
-            }
-        }
-    }
-    __shared__ int sred[2][4][32];
-    if (ACC_E || ACC_M) {
-        uint32_t ecnt[4][NLV], mcnt[4][NLM];
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-#pragma unroll
-            for (int l = 0; l < NLV; ++l) ecnt[k][l] = ACC_E ? ecb[(k * NLV + l) * BTS] : 0u;
-#pragma unroll
-            for (int l = 0; l < NLM; ++l) mcnt[k][l] = ACC_M ? mcb[(k * NLM + l) * BTS] : 0u;
-        }
-        for (int i = threadIdx.x; i < 2 * 4 * 32; i += BT) (&sred[0][0][0])[i] = 0;
         __syncthreads();
-        // all lanes of a block hold counters of its one quad: the 4 planes of a
-        // warp in one 32x32 transpose per counter level
-        if constexpr (ACC_E) {
-            int cnt[4];
-            packed_column_counts<NLV>(ecnt, lane, cnt);
+        const int k = threadIdx.x >> 5;
+        static_assert(kColourThreads == 128, "a warp per plane of the quad");
 #pragma unroll
-            for (int k = 0; k < 4; ++k) atomicAdd(&sred[0][k][lane], cnt[k]);
-        }
-        if constexpr (ACC_M) {
-            int cnt[4];
-            packed_column_counts<NLM>(mcnt, lane, cnt);
-#pragma unroll
-            for (int k = 0; k < 4; ++k) atomicAdd(&sred[1][k][lane], cnt[k]);
-        }
-        __syncthreads();
-        if (threadIdx.x < 128) {
-            const int k = threadIdx.x >> 5;
-            const size_t o = (((size_t)w * P.C + c) * P.T + 4 * q + k) * 32 + lane;
-            if constexpr (ACC_E) atomicAdd(&P.u_acc[o], sred[0][k][lane]);
-            if constexpr (ACC_M) atomicAdd(&P.up_acc[o], sred[1][k][lane]);
+        for (int c = 0; c < NC; ++c) {
+            const size_t o = (((size_t)w * P.C + c0 + c) * P.T + 4 * q + k) * 32 + lane;
+            if constexpr (ACC_E) atomicAdd(&P.u_acc[o], sred[c][0][k][lane]);
+            if constexpr (ACC_M) atomicAdd(&P.up_acc[o], sred[c][1][k][lane]);
         }
     }
 }

@@ -12,25 +12,25 @@
 namespace csg {
 
 
-// Launch shapes (measured at L=32 and L=48).  Plain colour launches: blocks of
-// kStreamThreads threads, kStreamSPT sites of the colour per thread.
-constexpr int kStreamThreads = 256;
-constexpr int kStreamSPT = 8;
-// Colour launches that count (energies, magnetisations) run smaller blocks of
-// kStreamAccSitesPerBlock sites (their counters live in shared memory, one
-// column per thread).
-constexpr int kStreamAccThreads = 128;
-#ifndef CSG_STREAM_ACC_SPT
-#define CSG_STREAM_ACC_SPT 8
-#endif
-constexpr int kStreamAccSPT = CSG_STREAM_ACC_SPT;
-constexpr int kStreamAccSitesPerBlock = kStreamAccThreads * kStreamAccSPT;
+// Colour launches: blocks of kColourThreads sites of a z-plane's half, walking
+// at most kColourMaxZ planes (colour_planes in csg_engine.cu chooses how many).
+constexpr int kColourThreads = 128;
+constexpr int kColourMaxZ = 16;
+constexpr int kStreamNLV = bit_length(6 * kColourMaxZ);  // bits of a per-thread bond count
+constexpr int kStreamNLM = bit_length(kColourMaxZ);      // bits of a per-thread site count
+// Copies of a temperature quad a colour launch's thread takes: both where it
+// only updates (shared bonds, thresholds and addresses); one where it counts,
+// since two sets of counters spill (L = 48: 139 against 120 us a launch).
 template <bool ACC>
-__host__ __device__ constexpr int colour_threads() { return ACC ? kStreamAccThreads : kStreamThreads; }
-template <bool ACC>
-__host__ __device__ constexpr int colour_spt() { return ACC ? kStreamAccSPT : kStreamSPT; }
-constexpr int kStreamNLV = bit_length(6 * kStreamAccSPT);  // bits of a per-thread bond count
-constexpr int kStreamNLM = bit_length(kStreamAccSPT);      // bits of a per-thread site count
+__host__ __device__ constexpr int colour_copies(int copies) { return ACC ? 1 : copies; }
+// Blocks per SM the colour kernel is built for, by the registers each variant
+// needs without spills that cost (a counting launch at 5 blocks, 96 registers:
+// 120 us at L = 48 and 42 at L = 32; at 4, 116 registers: 115 and 37).
+template <bool GEN_H, bool ACC_E, bool ACC_M, int NC>
+__host__ __device__ constexpr int colour_blocks() {
+    return ACC_E || ACC_M ? 4 : NC == 2 ? (GEN_H ? 4 : 5) : (GEN_H ? 6 : 7);
+}
+constexpr int kStreamThreads = 256;  // threads per block of the overlap passes
 // Overlap passes (both copies of every quad): blocks of kStreamThreads threads
 // over kOverlapSitesPerBlock sites (all N sites of a lattice).
 constexpr int kOverlapSPT = 8;
@@ -50,22 +50,11 @@ struct StreamParams {
     uint32_t* masks;  // [W][C][T] accepted-sample masks of the current round
     int* err;         // set to 1 by a sweep launch whose staging wait gave up
     int L, W, C, T, Q;
-    int nblk;   // blocks per quad of a counting colour launch
     int nblk2;  // blocks per quad of an overlap pass (over all N sites)
     uint32_t k0, k1, word0;
-    uint32_t mag_plane;  // ceil(2^32 / (L*L/2)): division by multiply-high
-    uint32_t mag_row;    // ceil(2^32 / (L/2))
     double H;
     PtTables tab;
 };
-
-// n / d for 0 <= n < L^3/2, d in {L/2, L*L/2}, with mag = ceil(2^32 / d): the
-// multiply-high estimate is never below n / d and at most one above it for
-// every even L <= 128 (checked exhaustively), so one correction makes it exact.
-__device__ __forceinline__ int div_magic(int n, int d, uint32_t mag) {
-    const int q = (int)__umulhi((uint32_t)n, mag);
-    return q - (q * d > n ? 1 : 0);
-}
 
 // The fused sweep launch (stream_sweep.cu): both colours of one sweep in one
 // pass over the state, for lattices whose ring of z-planes fits in shared
