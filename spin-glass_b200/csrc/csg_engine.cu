@@ -88,11 +88,13 @@ namespace {
 // change of a flip is dE = 12 - 4U + 2H(2s-1); the flip is accepted when a
 // 32-bit draw r satisfies r < floor(exp(-beta dE) 2^32), and always when
 // that value reaches 2^32 (dE <= 0).  ucut[t][s] is the first such U.
-// Returns whether the H=0 kernel (3 thresholds, U >= 3 always) describes the
-// table exactly.
-bool build_tables(const csg_config& cfg, csg::PtTables& tab) {
+// Returns the kernel variant the table needs (FieldMode in pt_kernel.cuh):
+// no field when the H = 0 rule (3 thresholds, U >= 3 always) describes it
+// exactly, a moderate one when spins down (s = 0) are always accepted from U =
+// 3 and spins up from U = 4 (0 < H < 2), else the general rule.
+int build_tables(const csg_config& cfg, csg::PtTables& tab) {
     std::memset(&tab, 0, sizeof(tab));
-    bool h0_exact = true;
+    bool h0_exact = true, moderate = true;
     for (int t = 0; t < cfg.dims.n_temps; ++t) {
         tab.beta[t] = cfg.betas[t];
         for (int s = 0; s < 2; ++s) {
@@ -105,38 +107,39 @@ bool build_tables(const csg_config& cfg, csg::PtTables& tab) {
                     if (cut == 7) cut = U;
                     tab.thr[t][s][U] = 0xFFFFFFFFu;
                 } else {
-                    if (cut != 7) h0_exact = false;  // non-monotone (cannot happen for beta >= 0)
+                    if (cut != 7) h0_exact = moderate = false;  // non-monotone (cannot happen for beta >= 0)
                     tab.thr[t][s][U] = (uint32_t)v;
                 }
             }
             tab.ucut[t][s] = (uint8_t)cut;
             if (cut != 3) h0_exact = false;
+            if (cut != 3 + s) moderate = false;
             // cut <= 3 (s = 0) and cut <= 5 (s = 1) for 0 <= H <= 4 (validate()),
             // as the general-field rule (flip_gen) requires
         }
         for (int U = 0; U < 3; ++U)
             if (tab.thr[t][0][U] != tab.thr[t][1][U]) h0_exact = false;
     }
-    return h0_exact && cfg.H == 0.0;
+    return h0_exact && cfg.H == 0.0 ? csg::kNoField : moderate ? csg::kModerateField : csg::kGeneralField;
 }
 
 using KernelFn = csg::ResidentFn;
 
-// The resident kernel for L (general-field variant when gen) with nseg column
+// The resident kernel for L (general-field variant when field) with nseg column
 // segments per thread; nullptr if that variant is not built.
-KernelFn select_kernel(int L, bool gen, int nseg) {
+KernelFn select_kernel(int L, int field, int nseg) {
     switch (L) {
-        case 4: return csg::resident_kernel_L4(gen, nseg);
-        case 6: return csg::resident_kernel_L6(gen, nseg);
-        case 8: return csg::resident_kernel_L8(gen, nseg);
-        case 10: return csg::resident_kernel_L10(gen, nseg);
-        case 12: return csg::resident_kernel_L12(gen, nseg);
-        case 14: return csg::resident_kernel_L14(gen, nseg);
-        case 16: return csg::resident_kernel_L16(gen, nseg);
-        case 18: return csg::resident_kernel_L18(gen, nseg);
-        case 20: return csg::resident_kernel_L20(gen, nseg);
-        case 22: return csg::resident_kernel_L22(gen, nseg);
-        case 24: return csg::resident_kernel_L24(gen, nseg);
+        case 4: return csg::resident_kernel_L4(field, nseg);
+        case 6: return csg::resident_kernel_L6(field, nseg);
+        case 8: return csg::resident_kernel_L8(field, nseg);
+        case 10: return csg::resident_kernel_L10(field, nseg);
+        case 12: return csg::resident_kernel_L12(field, nseg);
+        case 14: return csg::resident_kernel_L14(field, nseg);
+        case 16: return csg::resident_kernel_L16(field, nseg);
+        case 18: return csg::resident_kernel_L18(field, nseg);
+        case 20: return csg::resident_kernel_L20(field, nseg);
+        case 22: return csg::resident_kernel_L22(field, nseg);
+        case 24: return csg::resident_kernel_L24(field, nseg);
         default: return nullptr;
     }
 }
@@ -207,7 +210,7 @@ void fill_launch(cudaLaunchConfig_t& lc, cudaLaunchAttribute* attr, int W, const
 // times the quads per SM in a wave); ties go to the smaller cluster (fewer
 // cross-CTA exchanges), then to the default column split.  Fields of `forced`
 // (and of the process-wide override) that are non-zero fix that part.
-int make_plan(const csg_config& cfg, bool gen, Plan& out, PlanChoice forced = PlanChoice{}) {
+int make_plan(const csg_config& cfg, int field, Plan& out, PlanChoice forced = PlanChoice{}) {
     const int L = cfg.dims.L, W = cfg.dims.n_words;
     const int G = cfg.dims.n_copies * cfg.dims.n_temps / 4;
     if (use_stream(cfg)) {  // fixed launch shapes, nothing to plan
@@ -225,7 +228,7 @@ int make_plan(const csg_config& cfg, bool gen, Plan& out, PlanChoice forced = Pl
         }
         return CSG_OK;
     }
-    const bool has_m = gen || (cfg.flags & CSG_MEASURE_M);
+    const bool has_m = field != csg::kNoField || (cfg.flags & CSG_MEASURE_M);
     {
         std::lock_guard<std::mutex> lk(g_plan_mu);
         if (forced.qc == 0) forced.qc = g_override.quads_per_cta;
@@ -242,7 +245,7 @@ int make_plan(const csg_config& cfg, bool gen, Plan& out, PlanChoice forced = Pl
     for (int oi = 0; csg::nseg_option(L, oi) > 0; ++oi) {
         const int nseg = csg::nseg_option(L, oi);
         if (forced.nseg > 0 && nseg != forced.nseg) continue;
-        KernelFn fn = select_kernel(L, gen, nseg);
+        KernelFn fn = select_kernel(L, field, nseg);
         if (!fn) continue;
         for (int Qc = 1; Qc <= G; ++Qc) {
             if (G % Qc || (forced.qc > 0 && Qc != forced.qc)) continue;
@@ -252,8 +255,8 @@ int make_plan(const csg_config& cfg, bool gen, Plan& out, PlanChoice forced = Pl
             pl.NSEG = nseg;
             pl.TPQ = csg::threads_per_quad(L, nseg);
             pl.threads = (Qc * pl.TPQ + 31) / 32 * 32;
-            pl.smem = smem_for(L, Qc, has_m, gen);
-            if (pl.K > 16 || pl.smem > kMaxSmem || pl.threads > csg::max_cta_threads(gen, nseg))
+            pl.smem = smem_for(L, Qc, has_m, field != csg::kNoField);
+            if (pl.K > 16 || pl.smem > kMaxSmem || pl.threads > csg::max_cta_threads(field != csg::kNoField, nseg))
                 continue;
             if (prepare_kernel(fn, pl.smem, pl.K) != CSG_OK) continue;
             cudaLaunchConfig_t lc;
@@ -278,7 +281,7 @@ int make_plan(const csg_config& cfg, bool gen, Plan& out, PlanChoice forced = Pl
         return fail(CSG_ERR_UNSUPPORTED, forced.qc > 0 || forced.nseg > 0
                                              ? "plan override exceeds device limits"
                                              : "no launch plan fits this configuration");
-    return prepare_kernel(select_kernel(L, gen, out.NSEG), out.smem, out.K);
+    return prepare_kernel(select_kernel(L, field, out.NSEG), out.smem, out.K);
 }
 
 int64_t count_events(int64_t s0, int64_t n, int64_t k, int64_t first_sweep) {
@@ -289,9 +292,9 @@ int64_t count_events(int64_t s0, int64_t n, int64_t k, int64_t first_sweep) {
     return hi / k - (lo - 1) / k;
 }
 
-int fill_params(const csg_config& cfg, csg::PtParams& P, bool& gen) {
+int fill_params(const csg_config& cfg, csg::PtParams& P, int& field) {
     std::memset(&P, 0, sizeof(P));
-    gen = !build_tables(cfg, P.tab);
+    field = build_tables(cfg, P.tab);
     P.H = cfg.H;
     P.k0 = (uint32_t)cfg.seed;
     P.k1 = (uint32_t)(cfg.seed >> 32);
@@ -379,27 +382,31 @@ int colour_planes(const csg::StreamParams& S, int copies, int blocks_per_sm, int
 
 using ColourLaunch = void (*)(const csg::StreamParams&, int, int, long long, cudaStream_t);
 
-template <bool G, bool E, bool M, int C>
+template <int F, bool E, bool M, int C>
 void launch_colour(const csg::StreamParams& S, int nsm, int p, long long s, cudaStream_t st) {
     constexpr int NC = csg::colour_copies<E || M>(C);
-    const int zb = colour_planes(S, NC, csg::colour_blocks<G, E, M, NC>(), nsm, E || M);
+    const int zb = colour_planes(S, NC, csg::colour_blocks<F, E, M, NC>(), nsm, E || M);
     const int npb = (S.L * (S.L / 2) + csg::kColourThreads - 1) / csg::kColourThreads;
     const dim3 grid((unsigned)(S.W * (S.C / NC) * S.Q), (unsigned)(npb * ((S.L + zb - 1) / zb)));
-    launch_pdl(csg::stream_colour_kernel<G, E, M, NC>, grid, dim3(csg::kColourThreads), st, S, p, s, zb);
+    launch_pdl(csg::stream_colour_kernel<F, E, M, NC>, grid, dim3(csg::kColourThreads), st, S, p, s, zb);
+}
+
+template <int F, int C>
+ColourLaunch colour_launch_of(bool acc_e, bool acc_m) {
+    static const ColourLaunch fns[4] = {launch_colour<F, false, false, C>, launch_colour<F, false, true, C>,
+                                        launch_colour<F, true, false, C>, launch_colour<F, true, true, C>};
+    return fns[(acc_e ? 2 : 0) + (acc_m ? 1 : 0)];
 }
 
 template <int C>
-ColourLaunch colour_launch_of(bool gen, bool acc_e, bool acc_m) {
-    static const ColourLaunch fns[8] = {
-        launch_colour<false, false, false, C>, launch_colour<false, false, true, C>,
-        launch_colour<false, true, false, C>,  launch_colour<false, true, true, C>,
-        launch_colour<true, false, false, C>,  launch_colour<true, false, true, C>,
-        launch_colour<true, true, false, C>,   launch_colour<true, true, true, C>};
-    return fns[(gen ? 4 : 0) + (acc_e ? 2 : 0) + (acc_m ? 1 : 0)];
+ColourLaunch colour_launch_for(int field, bool acc_e, bool acc_m) {
+    return field == csg::kNoField         ? colour_launch_of<csg::kNoField, C>(acc_e, acc_m)
+           : field == csg::kModerateField ? colour_launch_of<csg::kModerateField, C>(acc_e, acc_m)
+                                          : colour_launch_of<csg::kGeneralField, C>(acc_e, acc_m);
 }
 
-ColourLaunch colour_launch(int copies, bool gen, bool acc_e, bool acc_m) {
-    return copies == 2 ? colour_launch_of<2>(gen, acc_e, acc_m) : colour_launch_of<1>(gen, acc_e, acc_m);
+ColourLaunch colour_launch(int copies, int field, bool acc_e, bool acc_m) {
+    return copies == 2 ? colour_launch_for<2>(field, acc_e, acc_m) : colour_launch_for<1>(field, acc_e, acc_m);
 }
 
 // Same schedule, Philox counters and arithmetic as the resident kernel's sweep
@@ -408,8 +415,8 @@ ColourLaunch colour_launch(int copies, bool gen, bool acc_e, bool acc_m) {
 int run_stream(const csg_config& cfg, uint32_t* spins, const uint32_t* bonds,
                const csg_device_obs* obs, int64_t sweep0, int64_t n_sweeps, cudaStream_t st) {
     csg::PtParams tp;
-    bool gen = false;
-    fill_params(cfg, tp, gen);
+    int field = csg::kNoField;
+    fill_params(cfg, tp, field);
     const csg_dims& d = cfg.dims;
     const StreamLayout lay = stream_layout(cfg);
     csg::StreamParams S;
@@ -476,13 +483,13 @@ int run_stream(const csg_config& cfg, uint32_t* spins, const uint32_t* bonds,
         const bool do_swap = sps > 0 && (s + 1) % sps == 0;
         const bool do_meas = spm > 0 && (s + 1) % spm == 0 && s >= cfg.sched.meas_start;
         const bool need_E = do_swap || do_meas;
-        const bool need_M = need_E && (gen || (do_meas && (cfg.flags & CSG_MEASURE_M)));
+        const bool need_M = need_E && (field != csg::kNoField || (do_meas && (cfg.flags & CSG_MEASURE_M)));
         if (fused) {
-            ce = csg::launch_stream_sweep(S, s, gen, need_E, need_M, st);
+            ce = csg::launch_stream_sweep(S, s, field != csg::kNoField, need_E, need_M, st);
             if (ce != cudaSuccess) break;
         } else {
-            colour_launch(d.n_copies, gen, false, need_M)(S, nsm, 0, s, st);
-            colour_launch(d.n_copies, gen, need_E, need_M)(S, nsm, 1, s, st);
+            colour_launch(d.n_copies, field, false, need_M)(S, nsm, 0, s, st);
+            colour_launch(d.n_copies, field, need_E, need_M)(S, nsm, 1, s, st);
         }
         if (need_E) {
             const long long round = do_swap ? (s + 1) / sps - 1 : 0;
@@ -529,15 +536,15 @@ int csg_detail::run_device(const csg_config& cfg, uint32_t* spins, const uint32_
         return run_stream(cfg, spins, bonds, obs, sweep0, n_sweeps, st);
     }
     csg::PtParams P;
-    bool gen = false;
-    fill_params(cfg, P, gen);
+    int field = csg::kNoField;
+    fill_params(cfg, P, field);
     Plan pl;
     if (plan_in)
         pl = *plan_in;  // planned before a stream capture
-    else if (int rc = make_plan(cfg, gen, pl, forced))
+    else if (int rc = make_plan(cfg, field, pl, forced))
         return rc;
     P.sweep_dev = sweep_dev;
-    KernelFn fn = select_kernel(cfg.dims.L, gen, pl.NSEG);
+    KernelFn fn = select_kernel(cfg.dims.L, field, pl.NSEG);
     if (!fn) return fail(CSG_ERR_UNSUPPORTED, "no resident kernel for this plan");
     P.spins = spins;
     P.bonds = bonds;
@@ -584,9 +591,9 @@ int csg_detail::chain_launch_starts(cudaGraph_t g, const std::vector<const csg_e
     std::vector<const void*> fns(members.size());
     for (size_t i = 0; i < members.size(); ++i) {
         csg::PtParams P;
-        bool gen = false;
-        fill_params(members[i]->cfg, P, gen);
-        fns[i] = reinterpret_cast<const void*>(select_kernel(members[i]->cfg.dims.L, gen, nseg[i]));
+        int field = csg::kNoField;
+        fill_params(members[i]->cfg, P, field);
+        fns[i] = reinterpret_cast<const void*>(select_kernel(members[i]->cfg.dims.L, field, nseg[i]));
     }
     size_t n = 0;
     CSG_CUDA(cudaGraphGetNodes(g, nullptr, &n));
@@ -625,16 +632,16 @@ std::vector<PlanChoice> csg_detail::plan_options(const csg_config& c) {
     std::vector<PlanChoice> out;
     if (use_stream(c)) return out;
     csg::PtParams P;
-    bool gen = false;
-    fill_params(c, P, gen);
+    int field = csg::kNoField;
+    fill_params(c, P, field);
     const int L = c.dims.L, G = c.dims.n_copies * c.dims.n_temps / 4;
-    const bool has_m = gen || (c.flags & CSG_MEASURE_M);
+    const bool has_m = field != csg::kNoField || (c.flags & CSG_MEASURE_M);
     for (int oi = 0; csg::nseg_option(L, oi) > 0; ++oi) {
         const int nseg = csg::nseg_option(L, oi);
         const int tpq = csg::threads_per_quad(L, nseg);
         for (int qc = 1; qc <= G; ++qc)
-            if (G % qc == 0 && G / qc <= 16 && smem_for(L, qc, has_m, gen) <= kMaxSmem &&
-                (qc * tpq + 31) / 32 * 32 <= csg::max_cta_threads(gen, nseg))
+            if (G % qc == 0 && G / qc <= 16 && smem_for(L, qc, has_m, field != csg::kNoField) <= kMaxSmem &&
+                (qc * tpq + 31) / 32 * 32 <= csg::max_cta_threads(field != csg::kNoField, nseg))
                 out.push_back(PlanChoice{qc, nseg});
     }
     return out;
@@ -642,12 +649,12 @@ std::vector<PlanChoice> csg_detail::plan_options(const csg_config& c) {
 
 int csg_detail::plan_engine(csg_engine* e, Plan& pl, size_t min_smem) {
     csg::PtParams P;
-    bool gen = false;
-    fill_params(e->cfg, P, gen);
-    if (int rc = make_plan(e->cfg, gen, pl, PlanChoice{e->qc, e->nseg})) return rc;
+    int field = csg::kNoField;
+    fill_params(e->cfg, P, field);
+    if (int rc = make_plan(e->cfg, field, pl, PlanChoice{e->qc, e->nseg})) return rc;
     if (pl.smem < min_smem && !use_stream(e->cfg)) {
         pl.smem = min_smem;
-        return prepare_kernel(select_kernel(e->cfg.dims.L, gen, pl.NSEG), pl.smem, pl.K);
+        return prepare_kernel(select_kernel(e->cfg.dims.L, field, pl.NSEG), pl.smem, pl.K);
     }
     return CSG_OK;
 }
@@ -794,10 +801,10 @@ int csg_detail::engine_create_pooled(const csg_config* cfg, cudaMemPool_t pool, 
     if (rc == CSG_OK) {
         // A launch plan must exist before the engine is handed out.
         csg::PtParams P;
-        bool gen = false;
-        fill_params(e->cfg, P, gen);
+        int field = csg::kNoField;
+        fill_params(e->cfg, P, field);
         Plan pl;
-        rc = make_plan(e->cfg, gen, pl);
+        rc = make_plan(e->cfg, field, pl);
     }
     if (rc != CSG_OK) {
         const std::string msg = last_error();
@@ -956,10 +963,10 @@ int csg_query_plan(const csg_config* cfg, csg_plan* out) {
     if (int rc = validate(cfg)) return rc;
     if (!out) return fail(CSG_ERR_ARG, "null output");
     csg::PtParams P;
-    bool gen = false;
-    fill_params(*cfg, P, gen);
+    int field = csg::kNoField;
+    fill_params(*cfg, P, field);
     Plan pl;
-    if (int rc = make_plan(*cfg, gen, pl)) return rc;
+    if (int rc = make_plan(*cfg, field, pl)) return rc;
     out->quads_per_cta = pl.Qc;
     out->ctas_per_word = pl.K;
     out->threads_per_quad = pl.TPQ;

@@ -12,11 +12,14 @@ namespace csg {
 namespace {
 
 template <int L, int I>
-ResidentFn pick(bool gen, int nseg) {
+ResidentFn pick(int field, int nseg) {
     constexpr int NS = nseg_option(L, I);
     if constexpr (NS > 0) {
-        if (nseg == NS) return gen ? pt_resident_kernel<L, true, NS> : pt_resident_kernel<L, false, NS>;
-        return pick<L, I + 1>(gen, nseg);
+        if (nseg == NS)
+            return field == kNoField         ? pt_resident_kernel<L, kNoField, NS>
+                   : field == kModerateField ? pt_resident_kernel<L, kModerateField, NS>
+                                             : pt_resident_kernel<L, kGeneralField, NS>;
+        return pick<L, I + 1>(field, nseg);
     } else {
         return nullptr;
     }
@@ -26,6 +29,6 @@ ResidentFn pick(bool gen, int nseg) {
 
 #define CSG_CAT2(a, b) a##b
 #define CSG_CAT(a, b) CSG_CAT2(a, b)
-ResidentFn CSG_CAT(resident_kernel_L, CSG_PT_L)(bool gen, int nseg) { return pick<CSG_PT_L, 0>(gen, nseg); }
+ResidentFn CSG_CAT(resident_kernel_L, CSG_PT_L)(int field, int nseg) { return pick<CSG_PT_L, 0>(field, nseg); }
 
 }  // namespace csg

@@ -32,6 +32,9 @@ __host__ __device__ constexpr int max_cta_threads(bool gen, int nseg) {
     return gen && nseg == 1 ? kMaxThreadsGenWalk : kMaxThreads;
 }
 
+// Which acceptance rule a kernel is built for (csg_engine.cu, build_tables).
+enum FieldMode { kNoField = 0, kModerateField = 1, kGeneralField = 2 };
+
 struct PtTables {
     double beta[kMaxT];
     uint32_t thr[kMaxT][2][7];  // acceptance thresholds, valid for U < ucut
@@ -320,6 +323,23 @@ __device__ __forceinline__ uint32_t flip_h0(uint32_t sa, uint32_t ca, uint32_t s
 // s ^ (x | y): the flipped spin word in one gate
 __device__ __forceinline__ uint32_t flipped(uint32_t s, const FlipTerms& f) { return lop3<0x1E>(s, f.x, f.y); }
 
+// A moderate field, 0 < H < 2: always accepted from U = 3 (spin down, s = 0) or
+// U = 4 (spin up).  With j thresholds of the spin's own above the draw (three
+// or four), j one more for spins down, a flip is accepted iff U + j >= 4.  The
+// masks A >= B >= C >= D of j >= 1..4 are selected by the spin; while D is not
+// set, j is A ^ B ^ C + 2B.  Thresholds as flip_gen takes them.  31 logic
+// instructions a word with the adders and Philox, where flip_gen takes 52.
+__device__ __forceinline__ FlipTerms flip_field_terms(uint32_t s0, uint32_t sa, uint32_t ca, uint32_t sb,
+                                                      uint32_t cb, uint32_t r, const uint4 ta, const uint4 tb) {
+    const uint32_t A = lop3<0xCF>(s0, below(r, tb.z), 0u);            // ~s0 | m
+    const uint32_t B = lop3<0xCA>(s0, below(r, tb.y), below(r, ta.z));  // s0 ? up : down
+    const uint32_t C = lop3<0xCA>(s0, below(r, tb.x), below(r, ta.y));
+    const uint32_t D = lop3<0xCA>(s0, below(r, ta.w), below(r, ta.x));
+    const uint32_t c = maj3(sa, sb, xor3(A, B, C));
+    const uint32_t o = lop3<0xFE>(ca, cb, B);  // any of the weight-2 terms
+    return FlipTerms{lop3<0xF8>(maj3(ca, cb, B), c, o), D};  // two of them, or one and the carry
+}
+
 // General field, 0 <= H <= 4.  A flip of centre spin s with U unsatisfied
 // bonds is accepted iff U >= ucut_s (dE <= 0) or the draw r < thr[s][U].
 // thr[s][U] does not decrease with U and is 0xFFFFFFFF from ucut_s on, and
@@ -381,9 +401,9 @@ struct SmemMap {
 using ResidentFn = void (*)(PtParams);
 
 // The resident kernel for lattice side L (each defined in its own translation
-// unit, pt_instances.cu built with CSG_PT_L = L): the general-field variant
-// when gen, with nseg column segments per thread; nullptr if not built.
-#define CSG_DECLARE_RESIDENT(LL) ResidentFn resident_kernel_L##LL(bool gen, int nseg);
+// unit, pt_instances.cu built with CSG_PT_L = L): for a FieldMode, with nseg
+// column segments per thread; nullptr if not built.
+#define CSG_DECLARE_RESIDENT(LL) ResidentFn resident_kernel_L##LL(int field, int nseg);
 CSG_DECLARE_RESIDENT(4)
 CSG_DECLARE_RESIDENT(6)
 CSG_DECLARE_RESIDENT(8)

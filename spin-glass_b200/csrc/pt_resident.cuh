@@ -84,9 +84,10 @@ __host__ __device__ constexpr int site_group(int zs) {
     return u;
 }
 
-template <int L, bool GEN_H, int NSEG>
-__global__ void __launch_bounds__(max_cta_threads(GEN_H, NSEG)) pt_resident_kernel(const __grid_constant__ PtParams P) {
+template <int L, int FIELD, int NSEG>
+__global__ void __launch_bounds__(max_cta_threads(FIELD != kNoField, NSEG)) pt_resident_kernel(const __grid_constant__ PtParams P) {
     using CF = Walk<L, NSEG>;
+    constexpr bool GEN_H = FIELD != kNoField;
     constexpr int N = CF::N, NH = CF::NH, LH = CF::LH, PL = CF::PL, NC = CF::NC, ZS = CF::ZS;
     constexpr int TPQ = CF::TPQ;
     constexpr int NLV = CF::NLV, NLD = CF::NLD, NLH = CF::NLH;
@@ -270,12 +271,16 @@ __global__ void __launch_bounds__(max_cta_threads(GEN_H, NSEG)) pt_resident_kern
                     const uint32_t sa = xor3(u0, u1, u2), ca = maj3(u0, u1, u2);
                     const uint32_t sb = xor3(u3, u4, u5), cb = maj3(u3, u4, u5);
                     uint32_t fl;
-                    if constexpr (GEN_H) {
+                    if constexpr (FIELD == kGeneralField) {
                         fl = flip_gen(s0, sa, ca, sb, cb, rr[kq], thrq[2 * kq], thrq[2 * kq + 1],
                                       (int)((uc0 >> (8 * kq)) & 0xFF), (int)((uc1 >> (8 * kq)) & 0xFF));
                         cw[kq] = s0 ^ fl;
                     } else {
-                        const FlipTerms ft = flip_h0_terms(sa, ca, sb, cb, rr[kq], th0[kq], th1[kq], th2[kq]);
+                        FlipTerms ft;
+                        if constexpr (FIELD == kModerateField)
+                            ft = flip_field_terms(s0, sa, ca, sb, cb, rr[kq], thrq[2 * kq], thrq[2 * kq + 1]);
+                        else
+                            ft = flip_h0_terms(sa, ca, sb, cb, rr[kq], th0[kq], th1[kq], th2[kq]);
                         fl = ft.x | ft.y;
                         cw[kq] = flipped(s0, ft);
                     }

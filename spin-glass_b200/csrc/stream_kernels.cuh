@@ -50,8 +50,8 @@ __device__ __forceinline__ void prefetch_l1(const void* a) {
 // that miss L1 in between.  256 samples, 2 copies, 32 temperatures, a launch:
 // L = 48, 97 -> 75 us (counting: 133 -> 115); L = 32, 29 -> 25 (47 -> 37)
 // against a thread per site with 7 loads and index arithmetic for each.
-template <bool GEN_H, bool ACC_E, bool ACC_M, int NC>
-__global__ void __launch_bounds__(kColourThreads, colour_blocks<GEN_H, ACC_E, ACC_M, NC>())
+template <int FIELD, bool ACC_E, bool ACC_M, int NC>
+__global__ void __launch_bounds__(kColourThreads, colour_blocks<FIELD, ACC_E, ACC_M, NC>())
     stream_colour_kernel(const __grid_constant__ StreamParams P, int p, long long s, int zb) {
     pdl_enter();
     constexpr int NLV = kStreamNLV, NLM = kStreamNLM;
@@ -163,14 +163,21 @@ __global__ void __launch_bounds__(kColourThreads, colour_blocks<GEN_H, ACC_E, AC
                     const uint32_t sa = xor3(u0, u1, u2), ca = maj3(u0, u1, u2);
                     const uint32_t sb = xor3(u3, u4, u5), cb = maj3(u3, u4, u5);
                     uint32_t fl;
-                    if constexpr (GEN_H) {
+                    if constexpr (FIELD == kGeneralField) {
                         uint4 ta, tb;
                         gen_thresholds(P.tab, 4 * q + k, ta, tb);
                         fl = flip_gen(s0, sa, ca, sb, cb, rr[k], ta, tb, P.tab.ucut[4 * q + k][0],
                                       P.tab.ucut[4 * q + k][1]);
                         cw[k] = s0 ^ fl;
                     } else {
-                        const FlipTerms ft = flip_h0_terms(sa, ca, sb, cb, rr[k], th0[k], th1[k], th2[k]);
+                        FlipTerms ft;
+                        if constexpr (FIELD == kModerateField) {
+                            uint4 ta, tb;
+                            gen_thresholds(P.tab, 4 * q + k, ta, tb);
+                            ft = flip_field_terms(s0, sa, ca, sb, cb, rr[k], ta, tb);
+                        } else {
+                            ft = flip_h0_terms(sa, ca, sb, cb, rr[k], th0[k], th1[k], th2[k]);
+                        }
                         fl = ft.x | ft.y;
                         cw[k] = flipped(s0, ft);
                     }

@@ -26,9 +26,9 @@ __host__ __device__ constexpr int colour_copies(int copies) { return ACC ? 1 : c
 // Blocks per SM the colour kernel is built for, by the registers each variant
 // needs without spills that cost (a counting launch at 5 blocks, 96 registers:
 // 120 us at L = 48 and 42 at L = 32; at 4, 116 registers: 115 and 37).
-template <bool GEN_H, bool ACC_E, bool ACC_M, int NC>
+template <int FIELD, bool ACC_E, bool ACC_M, int NC>
 __host__ __device__ constexpr int colour_blocks() {
-    return ACC_E || ACC_M ? 4 : NC == 2 ? (GEN_H ? 4 : 5) : (GEN_H ? 6 : 7);
+    return ACC_E || ACC_M ? 4 : NC == 2 ? (FIELD ? 4 : 5) : (FIELD ? 6 : 7);
 }
 constexpr int kStreamThreads = 256;  // threads per block of the overlap passes
 // Overlap passes (both copies of every quad): blocks of kStreamThreads threads
