@@ -18,6 +18,7 @@
 #include "philox.cuh"
 #include "pt_kernel.cuh"
 #include "aux_kernels.cuh"
+#include "checkpoint_kernels.cuh"
 #include "stream_kernels.cuh"
 
 namespace csg {
@@ -992,15 +993,37 @@ int csg_set_plan_override(const csg_plan* plan) {
 // ---------------------------------------------------------------------------
 namespace {
 
-size_t slot_of(int L, int x, int y, int z) {
-    const size_t N = (size_t)L * L * L;
-    return (size_t)((x + y + z) & 1) * (N / 2) + (size_t)(z * L + y) * (L / 2) + (size_t)(x >> 1);
-}
+// Device scratch of a call, in the order of the engine's stream.
+struct Scratch {
+    void* p = nullptr;
+    cudaStream_t st;
+    explicit Scratch(cudaStream_t s) : st(s) {}
+    Scratch(const Scratch&) = delete;
+    Scratch& operator=(const Scratch&) = delete;
+    ~Scratch() {
+        if (p) cudaFreeAsync(p, st);
+    }
+    int take(const csg_engine* e, size_t bytes) {
+        const cudaError_t ce = e->pool ? cudaMallocFromPoolAsync(&p, bytes, e->pool, st)
+                                       : cudaMallocAsync(&p, bytes, st);
+        if (ce == cudaSuccess) return CSG_OK;
+        cudaGetLastError();
+        p = nullptr;
+        return fail(CSG_ERR_NOMEM, std::string("checkpoint scratch: ") + cudaGetErrorString(ce));
+    }
+};
 
-size_t spin_at(const csg_dims& d, int w, int c, int t, size_t slot) {
-    const size_t N = (size_t)d.L * d.L * d.L;
-    return ((((size_t)w * d.n_copies + c) * (d.n_temps / 4) + (size_t)(t >> 2)) * N + slot) * 4 +
-           (size_t)(t & 3);
+// Scratch for the checkpoint of `words` words of samples at once (and extra
+// bytes): all of them up to 256 MB, fewer where the device cannot hold that.
+constexpr size_t kCheckpointScratch = (size_t)256 << 20;
+int checkpoint_scratch(const csg_engine* e, Scratch& sc, int& words, size_t extra) {
+    const csg_dims& d = e->cfg.dims;
+    const size_t word = (size_t)64 * d.L * d.L * d.L * 4;
+    words = (int)std::max<size_t>(1, std::min<size_t>(std::min(d.n_words, 32767), kCheckpointScratch / word));
+    for (;; words = (words + 1) / 2) {
+        const int rc = sc.take(e, words * word + extra);
+        if (rc == CSG_OK || words == 1) return rc;
+    }
 }
 
 }  // namespace
@@ -1069,33 +1092,19 @@ int csg_save_checkpoint(csg_engine* e, uint32_t* ref, size_t n_words) {
     const int L = d.L, W = d.n_words, T = d.n_temps;
     const size_t N = (size_t)L * L * L;
     if (n_words != (size_t)64 * W * N) return fail(CSG_ERR_ARG, "checkpoint size mismatch");
-    std::vector<uint32_t> sp(e->n_spins), bd(e->n_bonds);
-    if (int rc = csg_get_state(e, sp.data(), sp.size(), bd.data(), bd.size(), nullptr)) return rc;
-    for (int w = 0; w < W; ++w)
-        for (int z = 0; z < L; ++z)
-            for (int y = 0; y < L; ++y)
-                for (int x = 0; x < L; ++x) {
-                    const size_t si = slot_of(L, x, y, z), i = ((size_t)z * L + y) * L + x;
-                    const int xm = (x + L - 1) % L, ym = (y + L - 1) % L, zm = (z + L - 1) % L;
-                    const uint32_t f[6] = {bd[((size_t)w * 3 + 0) * N + slot_of(L, xm, y, z)],
-                                           bd[((size_t)w * 3 + 0) * N + si],
-                                           bd[((size_t)w * 3 + 1) * N + slot_of(L, x, ym, z)],
-                                           bd[((size_t)w * 3 + 1) * N + si],
-                                           bd[((size_t)w * 3 + 2) * N + slot_of(L, x, y, zm)],
-                                           bd[((size_t)w * 3 + 2) * N + si]};
-                    uint32_t sv[2][24];
-                    for (int c = 0; c < 2; ++c)
-                        for (int t = 0; t < T; ++t) sv[c][t] = sp[spin_at(d, w, c, t, si)];
-                    for (int b = 0; b < 32; ++b) {
-                        uint32_t jb = 0;
-                        for (int k = 0; k < 6; ++k) jb |= ((~f[k] >> b) & 1u) << (26 + k);
-                        for (int c = 0; c < 2; ++c) {
-                            uint32_t v = jb;
-                            for (int t = 0; t < T; ++t) v |= ((sv[c][t] >> b) & 1u) << t;
-                            ref[((size_t)2 * (32 * w + b) + c) * N + i] = v;
-                        }
-                    }
-                }
+    int step = 0;
+    Scratch sc(e->stream);
+    if (int rc = checkpoint_scratch(e, sc, step, 0)) return rc;
+    uint32_t* dev = static_cast<uint32_t*>(sc.p);
+    for (int w0 = 0; w0 < W; w0 += step) {
+        const int n = std::min(step, W - w0);
+        csg::checkpoint_save_kernel<<<dim3((unsigned)((N + 127) / 128), (unsigned)(2 * n)), 128, 0, e->stream>>>(
+            e->spins, e->bonds, csg::CheckpointDims{L, T, w0, n}, dev);
+        CSG_CUDA(cudaGetLastError());
+        CSG_CUDA(cudaMemcpyAsync(ref + (size_t)64 * w0 * N, dev, (size_t)64 * n * N * 4, cudaMemcpyDeviceToHost,
+                                 e->stream));
+    }
+    CSG_CUDA(cudaStreamSynchronize(e->stream));
     return CSG_OK;
 }
 
@@ -1107,38 +1116,41 @@ int csg_load_checkpoint(csg_engine* e, const uint32_t* ref, size_t n_words, int6
     const int L = d.L, W = d.n_words, T = d.n_temps;
     const size_t N = (size_t)L * L * L;
     if (n_words != (size_t)64 * W * N) return fail(CSG_ERR_ARG, "checkpoint size mismatch");
-    std::vector<uint32_t> sp(e->n_spins, 0u), bd(e->n_bonds, 0u);
-    for (int w = 0; w < W; ++w)
-        for (int z = 0; z < L; ++z)
-            for (int y = 0; y < L; ++y)
-                for (int x = 0; x < L; ++x) {
-                    const size_t si = slot_of(L, x, y, z), i = ((size_t)z * L + y) * L + x;
-                    const size_t nbi[3] = {((size_t)z * L + y) * L + (x + 1) % L,
-                                           ((size_t)z * L + (y + 1) % L) * L + x,
-                                           ((size_t)((z + 1) % L) * L + y) * L + x};
-                    uint32_t f[3] = {0, 0, 0};
-                    uint32_t sv[2][24] = {};
-                    for (int b = 0; b < 32; ++b) {
-                        const uint32_t v0 = ref[((size_t)2 * (32 * w + b)) * N + i];
-                        const uint32_t v1 = ref[((size_t)2 * (32 * w + b) + 1) * N + i];
-                        if ((v0 >> 26) != (v1 >> 26))
-                            return fail(CSG_ERR_STATE, "copies of a sample disagree on its bonds");
-                        for (int k = 0; k < 3; ++k) {
-                            const uint32_t vn = ref[((size_t)2 * (32 * w + b)) * N + nbi[k]];
-                            if (((v0 >> (27 + 2 * k)) & 1u) != ((vn >> (26 + 2 * k)) & 1u))
-                                return fail(CSG_ERR_STATE, "the two ends of a bond disagree");
-                            f[k] |= ((~v0 >> (27 + 2 * k)) & 1u) << b;
-                        }
-                        for (int t = 0; t < T; ++t) {
-                            sv[0][t] |= ((v0 >> t) & 1u) << b;
-                            sv[1][t] |= ((v1 >> t) & 1u) << b;
-                        }
-                    }
-                    for (int k = 0; k < 3; ++k) bd[((size_t)w * 3 + k) * N + si] = f[k];
-                    for (int c = 0; c < 2; ++c)
-                        for (int t = 0; t < T; ++t) sp[spin_at(d, w, c, t, si)] = sv[c][t];
-                }
-    return csg_set_state(e, sp.data(), sp.size(), bd.data(), bd.size(), sweep);
+    int step = 0;
+    Scratch sc(e->stream);
+    if (int rc = checkpoint_scratch(e, sc, step, 8)) return rc;
+    const size_t ref_bytes = (size_t)64 * step * N * 4;
+    uint32_t* dev = static_cast<uint32_t*>(sc.p);
+    auto* first = reinterpret_cast<unsigned long long*>(static_cast<char*>(sc.p) + ref_bytes);
+    const unsigned nb = (unsigned)((N + 127) / 128);
+    auto upload = [&](int w0, int n) {
+        return cudaMemcpyAsync(dev, ref + (size_t)64 * w0 * N, (size_t)64 * n * N * 4, cudaMemcpyHostToDevice,
+                               e->stream);
+    };
+    // check all of it before the engine's state is touched
+    CSG_CUDA(cudaMemsetAsync(first, 0xFF, 8, e->stream));
+    for (int w0 = 0; w0 < W; w0 += step) {
+        const int n = std::min(step, W - w0);
+        CSG_CUDA(upload(w0, n));
+        csg::checkpoint_check_kernel<<<dim3(nb, (unsigned)n), 128, 0, e->stream>>>(
+            dev, csg::CheckpointDims{L, T, w0, n}, first);
+        CSG_CUDA(cudaGetLastError());
+    }
+    unsigned long long bad = 0;
+    CSG_CUDA(cudaMemcpyAsync(&bad, first, 8, cudaMemcpyDeviceToHost, e->stream));
+    CSG_CUDA(cudaStreamSynchronize(e->stream));
+    if (bad != ~0ull)
+        return fail(CSG_ERR_STATE, bad & 1 ? "the two ends of a bond disagree" : "copies of a sample disagree on its bonds");
+    if (sweep < 0) return fail(CSG_ERR_ARG, "negative sweep index");
+    for (int w0 = 0; w0 < W; w0 += step) {
+        const int n = std::min(step, W - w0);
+        if (step < W) CSG_CUDA(upload(w0, n));  // else it is still there
+        csg::checkpoint_load_kernel<<<dim3(nb, (unsigned)(2 * n)), 128, 0, e->stream>>>(
+            dev, csg::CheckpointDims{L, T, w0, n}, e->spins, e->bonds);
+        CSG_CUDA(cudaGetLastError());
+    }
+    e->sweep = sweep;
+    return reset_obs(e);
 }
 
 }  // extern "C"
