@@ -200,10 +200,18 @@ __global__ void __launch_bounds__(max_cta_threads(FIELD != kNoField, NSEG)) pt_r
     const uint32_t site0 = (uint32_t)((z0 * L + cy) * L + 2 * ch);  // Philox word 0 without x & 1
 
     const long long sweep_base = P.sweep0 + (P.sweep_dev ? *P.sweep_dev : 0ll);
+    // sweeps until the next exchange and the next measurement (-1: never), and
+    // the round of the former: counted down, since 64-bit remainders by run-time
+    // divisors cost ~1000 cycles a sweep
+    int to_swap = P.sps > 0 ? P.sps - 1 - (int)(sweep_base % P.sps) : -1;
+    int to_meas = P.spm > 0 ? P.spm - 1 - (int)(sweep_base % P.spm) : -1;
+    long long round = P.sps > 0 ? sweep_base / P.sps : 0;
     for (int it = 0; it < P.n_sweeps; ++it) {
         const long long s = sweep_base + it;
-        const bool do_swap = P.sps > 0 && ((s + 1) % P.sps) == 0;
-        const bool do_meas = P.spm > 0 && ((s + 1) % P.spm) == 0 && s >= P.meas_start;
+        const bool do_swap = to_swap == 0;
+        const bool do_meas = to_meas == 0 && s >= P.meas_start;
+        to_swap = do_swap ? P.sps - 1 : to_swap - 1;
+        to_meas = to_meas == 0 ? P.spm - 1 : to_meas - 1;
         const bool need_E = do_swap || do_meas;
         const bool need_M = need_E && (GEN_H || (do_meas && (P.flags & kFlagMeasureM)));
         const uint32_t s32 = (uint32_t)s;
@@ -212,16 +220,13 @@ __global__ void __launch_bounds__(max_cta_threads(FIELD != kNoField, NSEG)) pt_r
         if (need_E)  // sE, sD and (if present) sM are contiguous
             for (int i = tid; i < Qc * 4 * 32 * (has_M ? 3 : 2); i += nthreads) sE[i] = 0;
 
-        uint32_t ecnt[4][NLV];
+        BondCounts<NLV> ecnt[4];
 #pragma unroll
-        for (int k = 0; k < 4; ++k)
-#pragma unroll
-            for (int l = 0; l < NLV; ++l) ecnt[k][l] = 0;
+        for (int k = 0; k < 4; ++k) ecnt[k].clear();
 
-        // one colour of the checkerboard; ACC: also add the post-flip
+        // one colour of the checkerboard; accum: also add the post-flip
         // unsatisfied-bond counts into the energy counters
-        auto colour_pass = [&](const int p, auto acc_tag) {
-            constexpr bool ACC = decltype(acc_tag)::value;
+        auto colour_pass = [&](const int p, const bool accum) {
             // x parity of the column's sites alternates along z: sites k = 0, 2, ...
             // have x = 2h + o0, sites k = 1, 3, ... x = 2h + 1 - o0
             const int o0 = (cy + z0 + p) & 1;
@@ -243,10 +248,8 @@ __global__ void __launch_bounds__(max_cta_threads(FIELD != kNoField, NSEG)) pt_r
             const uint32_t* const FoZ = Fo + 2 * N;
             const uint32_t iE = site0 + (uint32_t)o0, iO = site0 + (uint32_t)(1 - o0);
 
-            // site k of the column (odd: k & 1; dzm, dzp: z-neighbour offsets);
-            // wd receives the post-flip full-adder words for the energy counters
-            auto site = [&](const int k, const bool odd, const int dzm, const int dzp,
-                            uint32_t (&wd)[4][4]) {
+            // site k of the column (odd: k & 1; dzm, dzp: z-neighbour offsets)
+            auto site = [&](const int k, const bool odd, const int dzm, const int dzp) {
                 const int off = k * PL;
                 const uint4 cv = ld4(Sc, off);
                 const uint4 a0 = ld4(odd ? SoXmO : SoXmE, off);
@@ -262,6 +265,7 @@ __global__ void __launch_bounds__(max_cta_threads(FIELD != kNoField, NSEG)) pt_r
                 const uint32_t n0w[4] = {a0.x, a0.y, a0.z, a0.w}, n1w[4] = {a1.x, a1.y, a1.z, a1.w};
                 const uint32_t n2w[4] = {a2.x, a2.y, a2.z, a2.w}, n3w[4] = {a3.x, a3.y, a3.z, a3.w};
                 const uint32_t n4w[4] = {a4.x, a4.y, a4.z, a4.w}, n5w[4] = {a5.x, a5.y, a5.z, a5.w};
+                uint32_t wa[4], wb[4], wc[4], wd[4], wf[4];  // adders and flips, for the counters
 #pragma unroll
                 for (int kq = 0; kq < 4; ++kq) {
                     const uint32_t s0 = cw[kq];
@@ -284,36 +288,30 @@ __global__ void __launch_bounds__(max_cta_threads(FIELD != kNoField, NSEG)) pt_r
                         fl = ft.x | ft.y;
                         cw[kq] = flipped(s0, ft);
                     }
-                    if constexpr (ACC) {
-                        wd[kq][0] = sa ^ fl;
-                        wd[kq][1] = sb ^ fl;
-                        wd[kq][2] = ca ^ fl;
-                        wd[kq][3] = cb ^ fl;
-                    }
+                    wa[kq] = sa;
+                    wb[kq] = sb;
+                    wc[kq] = ca;
+                    wd[kq] = cb;
+                    wf[kq] = fl;
                 }
                 st4(Sc, off, make_uint4(cw[0], cw[1], cw[2], cw[3]));
-            };
-            auto acc2 = [&](const uint32_t (&wa)[4][4], const uint32_t (&wb)[4][4]) {
-                if constexpr (ACC) {
+                if (accum) {
 #pragma unroll
-                    for (int kq = 0; kq < 4; ++kq)
-                        vc_add_2sites<NLV>(ecnt[kq], wa[kq][0], wa[kq][1], wa[kq][2], wa[kq][3],
-                                           wb[kq][0], wb[kq][1], wb[kq][2], wb[kq][3]);
+                    for (int kq = 0; kq < 4; ++kq) {
+                        if (odd)
+                            ecnt[kq].add_odd(wa[kq], wb[kq], wc[kq], wd[kq], wf[kq]);
+                        else
+                            ecnt[kq].add_even(wa[kq], wb[kq], wc[kq], wd[kq], wf[kq]);
+                    }
                 }
             };
             if constexpr (ZS <= kUnrollAllZS) {
 #pragma unroll
-                for (int k = 0; k < ZS; k += 2) {
-                    uint32_t wa[4][4], wb[4][4];
-                    site(k, false, k == 0 ? dzF : -PL, k == ZS - 1 ? dzL : PL, wa);
-                    if (k + 1 < ZS) {
-                        site(k + 1, true, -PL, k + 1 == ZS - 1 ? dzL : PL, wb);
-                        acc2(wa, wb);
-                    } else if constexpr (ACC) {
+                for (int k = 0; k < ZS; ++k)
+                    site(k, (k & 1) != 0, k == 0 ? dzF : -PL, k == ZS - 1 ? dzL : PL);
+                if (ZS % 2 == 1 && accum) {
 #pragma unroll
-                        for (int kq = 0; kq < 4; ++kq)
-                            vc_add_site<NLV>(ecnt[kq], wa[kq][0], wa[kq][1], wa[kq][2], wa[kq][3]);
-                    }
+                    for (int kq = 0; kq < 4; ++kq) ecnt[kq].finish_even();
                 }
             } else {
                 // a group's sites sit at fixed offsets from its first one; only
@@ -327,28 +325,36 @@ __global__ void __launch_bounds__(max_cta_threads(FIELD != kNoField, NSEG)) pt_r
                     const int dzpL = k0 + U == ZS ? dzL : PL;
 #pragma unroll
                     for (int u = 0; u < U; u += 2) {
-                        uint32_t wa[4][4], wb[4][4];
-                        site(k0 + u, false, u == 0 ? dzm0 : -PL, PL, wa);
-                        site(k0 + u + 1, true, -PL, u + 2 == U ? dzpL : PL, wb);
-                        acc2(wa, wb);
+                        site(k0 + u, false, u == 0 ? dzm0 : -PL, PL);
+                        site(k0 + u + 1, true, -PL, u + 2 == U ? dzpL : PL);
                     }
                 }
             }
         };
-        if (active) colour_pass(0, std::false_type{});
+        // three copies of the pass, two of them without the counting code (one
+        // copy for both colours, counting under a branch, is 5 % slower where
+        // nothing counts and 3 % where every sweep does)
+        if (active) colour_pass(0, false);
         __syncthreads();
         if (active) {
             if (need_E)
-                colour_pass(1, std::true_type{});
+                colour_pass(1, true);
             else
-                colour_pass(1, std::false_type{});
+                colour_pass(1, false);
         }
         __syncthreads();
 
         if (!need_E) continue;
 
         // ---- per-sample unsatisfied-bond totals of this CTA's planes ----
-        add_plane_counts<NLV>(ecnt, jt, Qc, lane, [&](int jj) { return sE + jj * 4 * 32; });
+        {
+            uint32_t v[4][NLV];
+#pragma unroll
+            for (int k = 0; k < 4; ++k)
+#pragma unroll
+                for (int l = 0; l < NLV; ++l) v[k][l] = ecnt[k].v[l];
+            add_plane_counts<NLV>(v, jt, Qc, lane, [&](int jj) { return sE + jj * 4 * 32; });
+        }
         if (need_M) {
             uint32_t mc[4][NLD];
 #pragma unroll
@@ -373,7 +379,6 @@ __global__ void __launch_bounds__(max_cta_threads(FIELD != kNoField, NSEG)) pt_r
         // readers below complete them
         uint32_t mask_keep = 0;  // exchange mask word this thread later finds in sD
         if (do_swap) {
-            const long long round = (s + 1) / P.sps - 1;
             const int par = (int)(round & 1);
             // the uniform of this lane for the warp's first pair does not depend
             // on the energies: draw it while the cluster barrier is pending
@@ -509,6 +514,7 @@ __global__ void __launch_bounds__(max_cta_threads(FIELD != kNoField, NSEG)) pt_r
             // measurement then reads the other copy's planes, perhaps remote
             if (par || do_meas) cluster.sync();
             else __syncthreads();
+            ++round;
         } else {
             __syncthreads();
         }

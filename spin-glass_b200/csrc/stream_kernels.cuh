@@ -69,13 +69,13 @@ __global__ void __launch_bounds__(kColourThreads, colour_blocks<FIELD, ACC_E, AC
     const int i = pb * kColourThreads + threadIdx.x;  // (y, h) of the plane's half
     const bool active = i < PL;
 
-    uint32_t ecnt[NC][4][NLV], mcnt[NC][4][NLM];
+    BondCounts<NLV> ecnt[NC][4];
+    uint32_t mcnt[NC][4][NLM];
 #pragma unroll
     for (int c = 0; c < NC; ++c)
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
-#pragma unroll
-            for (int l = 0; l < NLV; ++l) ecnt[c][k][l] = 0;
+            ecnt[c][k].clear();
 #pragma unroll
             for (int l = 0; l < NLM; ++l) mcnt[c][k][l] = 0;
         }
@@ -123,7 +123,7 @@ __global__ void __launch_bounds__(kColourThreads, colour_blocks<FIELD, ACC_E, AC
             zm[c] = *elem(Sq + c * copy + (size_t)(z0 == 0 ? L - 1 : z0 - 1) * PL, oo);
             zcur[c] = *elem(Sq + c * copy + (size_t)z0 * PL, oo);
         }
-        auto update_site = [&](const int z, const bool odd, uint32_t (&wd)[NC][4][4]) {
+        auto update_site = [&](const int z, const bool odd) {
             // the lines of the next two planes that no earlier load of this
             // block brought in: on their way while this site is updated
             // (L = 48: 75.0 us a launch instead of 79.5)
@@ -183,10 +183,10 @@ __global__ void __launch_bounds__(kColourThreads, colour_blocks<FIELD, ACC_E, AC
                     }
                     // post-flip unsatisfied bonds (energy) and spins up, counted at once
                     if constexpr (ACC_E) {
-                        wd[c][k][0] = sa ^ fl;
-                        wd[c][k][1] = sb ^ fl;
-                        wd[c][k][2] = ca ^ fl;
-                        wd[c][k][3] = cb ^ fl;
+                        if (odd)
+                            ecnt[c][k].add_odd(sa, sb, ca, cb, fl);
+                        else
+                            ecnt[c][k].add_even(sa, sb, ca, cb, fl);
                     }
                     if constexpr (ACC_M) {
                         uint32_t carry = cw[k];
@@ -205,17 +205,8 @@ __global__ void __launch_bounds__(kColourThreads, colour_blocks<FIELD, ACC_E, AC
         };
 #pragma unroll 1
         for (int z = z0; z < z1; z += 2) {  // L and zb are even
-            uint32_t wa[NC][4][4], wb[NC][4][4];
-            update_site(z, false, wa);
-            update_site(z + 1, true, wb);
-            if constexpr (ACC_E) {
-#pragma unroll
-                for (int c = 0; c < NC; ++c)
-#pragma unroll
-                    for (int k = 0; k < 4; ++k)
-                        vc_add_2sites<NLV>(ecnt[c][k], wa[c][k][0], wa[c][k][1], wa[c][k][2], wa[c][k][3],
-                                           wb[c][k][0], wb[c][k][1], wb[c][k][2], wb[c][k][3]);
-            }
+            update_site(z, false);
+            update_site(z + 1, true);
         }
     }
     if constexpr (ACC_E || ACC_M) {
@@ -228,7 +219,12 @@ __global__ void __launch_bounds__(kColourThreads, colour_blocks<FIELD, ACC_E, AC
             // a warp in one 32x32 transpose per counter level
             int cnt[4];
             if constexpr (ACC_E) {
-                packed_column_counts<NLV>(ecnt[c], lane, cnt);
+                uint32_t v[4][NLV];
+#pragma unroll
+                for (int k = 0; k < 4; ++k)
+#pragma unroll
+                    for (int l = 0; l < NLV; ++l) v[k][l] = ecnt[c][k].v[l];
+                packed_column_counts<NLV>(v, lane, cnt);
 #pragma unroll
                 for (int k = 0; k < 4; ++k) atomicAdd(&sred[c][0][k][lane], cnt[k]);
             }
