@@ -262,7 +262,7 @@ int csg_batch_set_member_plan(csg_batch* b, int32_t i, const csg_plan* plan) {
     const int nseg = tpq > 0 ? tpq / (L * (L / 2)) : 0;
     if (tpq > 0 && nseg * L * (L / 2) != tpq) return fail(CSG_ERR_ARG, "threads_per_quad is not L*L/2*s");
     bool ok = qc == 0 && nseg == 0;
-    for (const PlanChoice& o : plan_options(e->cfg))
+    for (const PlanChoice& o : plan_options(e->cfg, false))
         if ((qc == 0 || o.qc == qc) && (nseg == 0 || o.nseg == nseg)) ok = true;
     if (!ok) return fail(CSG_ERR_UNSUPPORTED, "no built tile with these quads per CTA and threads per quad");
     e->qc = qc;
@@ -340,7 +340,7 @@ int csg_batch_tune(csg_batch* b, int64_t probe_sweeps, int32_t* chosen) {
     std::vector<std::vector<PlanChoice>> options(n);
     size_t combos = 1;
     for (size_t i = 0; i < n; ++i) {
-        options[i] = plan_options(b->eng[i]->cfg);
+        options[i] = plan_options(b->eng[i]->cfg, true);
         combos *= std::max<size_t>(1, options[i].size());
     }
     auto set_choice = [&](size_t i, const PlanChoice& pc) {

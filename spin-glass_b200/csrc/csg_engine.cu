@@ -5,6 +5,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <array>
 #include <cmath>
 #include <cstring>
 #include <mutex>
@@ -205,12 +206,42 @@ void fill_launch(cudaLaunchConfig_t& lc, cudaLaunchAttribute* attr, int W, const
     lc.numAttrs = 2;
 }
 
+// Time of one sweep of a CTA's SM, in cycles: every thread walks its ZS sites of
+// each colour; a round of one site per warp takes the latency of a site for
+// one warp a scheduler and the issue of all of them for more, and a sweep with an
+// exchange or a measurement costs every warp its share of the reductions.
+// Fitted to every tile of 27 shapes, L = 4..24 (with one word of 16
+// temperatures at L = 12, us a sweep: 72 threads a quad 5.6, 144 4.2, 288 3.3, 432
+// 3.1; with exchange and measurement 12.6, 9.8, 8.8, 8.6).
+long sweep_cycles(const csg_config& cfg, int zs, int warps) {
+    const int wps = (warps + 3) / 4;
+    const long site = wps == 1 ? 467 : wps == 2 ? 620 : wps == 3 ? 860 : 283L * wps;
+    const csg_schedule& sc = cfg.sched;
+    long every = 0;  // sweeps between two that reduce
+    if (sc.sweeps_per_swap > 0) every = sc.sweeps_per_swap;
+    if (sc.sweeps_per_meas > 0 && (every == 0 || sc.sweeps_per_meas < every)) every = sc.sweeps_per_meas;
+    return 2L * zs * site + (every > 0 ? 250L * warps / every : 0);
+}
+
+// Plans chosen before, by everything the choice depends on: planning asks the
+// runtime for the occupancy of every candidate (~2 us each), which is most of
+// what a short call costs on the host.
+struct PlanKey {
+    int v[14];
+    bool operator==(const PlanKey& o) const { return std::memcmp(v, o.v, sizeof(v)) == 0; }
+};
+struct PlanCache {
+    static constexpr size_t kMost = 64;
+    std::vector<std::pair<PlanKey, Plan>> entries;  // under g_plan_mu
+};
+PlanCache g_plans;
+
 // Launch plan: split the G = C*T/4 quads of a word over K = G/Qc CTAs of a
-// cluster, each quad's team of TPQ = L * L/2 * NSEG threads.  The score is the
-// number of quads the busiest SM must sweep (waves of co-resident clusters
-// times the quads per SM in a wave); ties go to the smaller cluster (fewer
-// cross-CTA exchanges), then to the default column split.  Fields of `forced`
-// (and of the process-wide override) that are non-zero fix that part.
+// cluster, each quad's team of TPQ = L * L/2 * NSEG threads.  First the fewest
+// quads on the busiest SM (waves of co-resident clusters times the quads per
+// SM in a wave), then the smaller cluster (fewer cross-CTA exchanges), then the
+// column split with the shortest sweep.  Fields of `forced` (and of the
+// process-wide override) that are non-zero fix that part.
 int make_plan(const csg_config& cfg, int field, Plan& out, PlanChoice forced = PlanChoice{}) {
     const int L = cfg.dims.L, W = cfg.dims.n_words;
     const int G = cfg.dims.n_copies * cfg.dims.n_temps / 4;
@@ -229,7 +260,10 @@ int make_plan(const csg_config& cfg, int field, Plan& out, PlanChoice forced = P
         }
         return CSG_OK;
     }
-    const bool has_m = field != csg::kNoField || (cfg.flags & CSG_MEASURE_M);
+    const bool gen = field != csg::kNoField;
+    const bool has_m = gen || (cfg.flags & CSG_MEASURE_M);
+    int dev = 0, nsm = 0;
+    CSG_CUDA(cudaGetDevice(&dev));
     {
         std::lock_guard<std::mutex> lk(g_plan_mu);
         if (forced.qc == 0) forced.qc = g_override.quads_per_cta;
@@ -239,10 +273,21 @@ int make_plan(const csg_config& cfg, int field, Plan& out, PlanChoice forced = P
     if (forced.qc < 0 || forced.nseg < 0) return fail(CSG_ERR_ARG, "negative plan entry");
     if (forced.qc > 0 && G % forced.qc != 0)
         return fail(CSG_ERR_ARG, "plan override does not divide the quads");
-    int dev = 0, nsm = 0;
-    CSG_CUDA(cudaGetDevice(&dev));
+    const PlanKey key = {{dev, L, W, G, cfg.dims.n_copies, field, has_m, cfg.sched.sweeps_per_swap,
+                          cfg.sched.sweeps_per_meas, forced.qc, forced.nseg, 0, 0, 0}};
+    bool known = false;
+    {
+        std::lock_guard<std::mutex> lk(g_plan_mu);
+        for (const auto& e : g_plans.entries)
+            if (e.first == key) {
+                out = e.second;
+                known = true;
+                break;
+            }
+    }
+    if (known) return prepare_kernel(select_kernel(L, field, out.NSEG), out.smem, out.K);
     CSG_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
-    long best = -1;
+    std::array<long, 4> best = {-1, 0, 0, 0};
     for (int oi = 0; csg::nseg_option(L, oi) > 0; ++oi) {
         const int nseg = csg::nseg_option(L, oi);
         if (forced.nseg > 0 && nseg != forced.nseg) continue;
@@ -256,8 +301,8 @@ int make_plan(const csg_config& cfg, int field, Plan& out, PlanChoice forced = P
             pl.NSEG = nseg;
             pl.TPQ = csg::threads_per_quad(L, nseg);
             pl.threads = (Qc * pl.TPQ + 31) / 32 * 32;
-            pl.smem = smem_for(L, Qc, has_m, field != csg::kNoField);
-            if (pl.K > 16 || pl.smem > kMaxSmem || pl.threads > csg::max_cta_threads(field != csg::kNoField, nseg))
+            pl.smem = smem_for(L, Qc, has_m, gen);
+            if (pl.K > 16 || pl.smem > kMaxSmem || pl.threads > csg::max_cta_threads(gen, nseg))
                 continue;
             if (prepare_kernel(fn, pl.smem, pl.K) != CSG_OK) continue;
             cudaLaunchConfig_t lc;
@@ -269,19 +314,24 @@ int make_plan(const csg_config& cfg, int field, Plan& out, PlanChoice forced = P
                 continue;
             }
             const long waves = (W + nclusters - 1) / nclusters;
-            const long per_wave = (long)std::min(W, nclusters) * pl.K;
-            const long load = waves * ((per_wave + nsm - 1) / nsm) * Qc;
-            const long score = (load * 64 + pl.K) * 8 + oi;
-            if (best < 0 || score < best) {
+            const long per_sm = ((long)std::min(W, nclusters) * pl.K + nsm - 1) / nsm;
+            const std::array<long, 4> score = {waves * per_sm * Qc, pl.K,
+                                               sweep_cycles(cfg, L / nseg, (int)per_sm * pl.threads / 32), oi};
+            if (best[0] < 0 || score < best) {
                 best = score;
                 out = pl;
             }
         }
     }
-    if (best < 0)
+    if (best[0] < 0)
         return fail(CSG_ERR_UNSUPPORTED, forced.qc > 0 || forced.nseg > 0
                                              ? "plan override exceeds device limits"
                                              : "no launch plan fits this configuration");
+    {
+        std::lock_guard<std::mutex> lk(g_plan_mu);
+        if (g_plans.entries.size() >= PlanCache::kMost) g_plans.entries.clear();
+        g_plans.entries.push_back({key, out});
+    }
     return prepare_kernel(select_kernel(L, field, out.NSEG), out.smem, out.K);
 }
 
@@ -629,7 +679,7 @@ int csg_detail::chain_launch_starts(cudaGraph_t g, const std::vector<const csg_e
     return CSG_OK;
 }
 
-std::vector<PlanChoice> csg_detail::plan_options(const csg_config& c) {
+std::vector<PlanChoice> csg_detail::plan_options(const csg_config& c, bool tuned) {
     std::vector<PlanChoice> out;
     if (use_stream(c)) return out;
     csg::PtParams P;
@@ -637,7 +687,7 @@ std::vector<PlanChoice> csg_detail::plan_options(const csg_config& c) {
     fill_params(c, P, field);
     const int L = c.dims.L, G = c.dims.n_copies * c.dims.n_temps / 4;
     const bool has_m = field != csg::kNoField || (c.flags & CSG_MEASURE_M);
-    for (int oi = 0; csg::nseg_option(L, oi) > 0; ++oi) {
+    for (int oi = 0; csg::nseg_option(L, oi) > 0 && (!tuned || oi < csg::tuned_splits(L)); ++oi) {
         const int nseg = csg::nseg_option(L, oi);
         const int tpq = csg::threads_per_quad(L, nseg);
         for (int qc = 1; qc <= G; ++qc)

@@ -81,8 +81,9 @@ CSG_INTERNAL bool use_stream(const csg_config& c);  // streaming engine, not the
 CSG_INTERNAL size_t footprint_bytes(const csg_config& c);
 
 // The (quads per CTA, column segments) pairs that fit one CTA and one
-// cluster of the resident kernel (empty for the streaming engine).
-CSG_INTERNAL std::vector<PlanChoice> plan_options(const csg_config& c);
+// cluster of the resident kernel (empty for the streaming engine); tuned: only
+// the column splits worth trying on a full GPU.
+CSG_INTERNAL std::vector<PlanChoice> plan_options(const csg_config& c, bool tuned);
 
 // Plan of an engine's resident kernel (its tuner choice e->qc / e->nseg, if
 // any), with the CTA's shared memory raised to at least min_smem.

@@ -107,15 +107,23 @@ struct Walk {
     static_assert(TPQ >= 32, "a warp spans at most two quads");
 };
 
-// Column segments per thread the resident kernel is built with, for each L:
-// the first entry is the default, the second (if any) a team twice as large
-// with half as many sites per thread.
+// Column splits (segments per column) the resident kernel is built with, for
+// each L.  The first entry is the default; the first tuned_splits(L) are the
+// ones a full GPU may want (and the batch tuner tries), the others are larger
+// teams that pay where an SM has few quads (make_plan weighs them all).
 __host__ __device__ constexpr int nseg_option(int L, int i) {
     return L == 4 ? (i == 0 ? 4 : 0)
-         : L == 6 ? (i == 0 ? 2 : 0)
-         : L <= 16 ? (i == 0 ? (L <= 10 ? 2 : 1) : i == 1 ? (L <= 10 ? 1 : 2) : 0)
+         : L == 6 ? (i == 0 ? 2 : i == 1 ? 6 : 0)
+         : L == 8 ? (i == 0 ? 2 : i == 1 ? 1 : i == 2 ? 4 : i == 3 ? 8 : 0)
+         : L == 10 ? (i == 0 ? 2 : i == 1 ? 1 : i == 2 ? 5 : 0)
+         : L == 12 ? (i == 0 ? 1 : i == 1 ? 2 : i == 2 ? 4 : i == 3 ? 6 : 0)
+         : L == 14 ? (i == 0 ? 1 : i == 1 ? 2 : 0)
+         : L == 16 ? (i == 0 ? 1 : i == 1 ? 2 : i == 2 ? 4 : 0)
+         : L == 18 ? (i == 0 ? 1 : i == 1 ? 3 : 0)
+         : L == 20 ? (i == 0 ? 1 : i == 1 ? 2 : 0)
          : (i == 0 ? 1 : 0);
 }
+__host__ __device__ constexpr int tuned_splits(int L) { return L >= 8 && L <= 16 ? 2 : 1; }
 __host__ __device__ constexpr int threads_per_quad(int L, int nseg) { return L * (L / 2) * nseg; }
 
 // One three-input logic instruction with truth table LUT (a = 0xF0, b = 0xCC,

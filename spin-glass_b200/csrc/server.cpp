@@ -30,7 +30,7 @@ namespace {
 // cluster barriers per unit of work); automatic (the single-request plan) for
 // the streaming engine.
 PlanChoice shared_gpu_plan(const csg_config& c) {
-    const std::vector<PlanChoice> opts = plan_options(c);
+    const std::vector<PlanChoice> opts = plan_options(c, true);
     PlanChoice best{};
     for (const PlanChoice& o : opts)
         if (o.nseg == opts.front().nseg && o.qc > best.qc) best = o;
