@@ -48,6 +48,88 @@ using namespace csg_detail;
 
 namespace {
 
+constexpr uint64_t kScratchKept = (uint64_t)64 << 20;
+
+// The scratch pool of one device context.  The context is known by its id, so
+// that a pool of a context that was torn down is never touched again.
+struct ScratchPool {
+    int dev;
+    unsigned long long ctx;
+    cudaMemPool_t pool;
+};
+std::mutex g_scratch_mu;
+std::vector<ScratchPool> g_scratch;
+
+bool current_context(int* dev, unsigned long long* id) {
+    using GetId = int (*)(void*, unsigned long long*);  // cuCtxGetId of the driver
+    static const GetId get = [] {
+        void* fn = nullptr;
+        cudaDriverEntryPointQueryResult found = cudaDriverEntryPointSymbolNotFound;
+        if (cudaGetDriverEntryPoint("cuCtxGetId", &fn, cudaEnableDefault, &found) != cudaSuccess ||
+            found != cudaDriverEntryPointSuccess) {
+            cudaGetLastError();
+            fn = nullptr;
+        }
+        return reinterpret_cast<GetId>(fn);
+    }();
+    if (!get || cudaGetDevice(dev) != cudaSuccess) return false;
+    return get(nullptr, id) == 0;
+}
+
+// The pool of the current context; nullptr where there is none (make: unless it
+// can be made).
+cudaMemPool_t scratch_pool(bool make) {
+    int dev = 0;
+    unsigned long long ctx = 0;
+    if (!current_context(&dev, &ctx)) return nullptr;
+    std::lock_guard<std::mutex> lk(g_scratch_mu);
+    for (size_t i = 0; i < g_scratch.size(); ++i) {
+        if (g_scratch[i].dev != dev) continue;
+        if (g_scratch[i].ctx == ctx) return g_scratch[i].pool;
+        g_scratch.erase(g_scratch.begin() + (long)i);  // went with its context
+        break;
+    }
+    if (!make) return nullptr;
+    cudaMemPoolProps props = {};
+    props.allocType = cudaMemAllocationTypePinned;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = dev;
+    cudaMemPool_t pool = nullptr;
+    uint64_t keep = kScratchKept;
+    if (cudaMemPoolCreate(&pool, &props) != cudaSuccess) {
+        cudaGetLastError();
+        return nullptr;
+    }
+    if (cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep) != cudaSuccess) cudaGetLastError();
+    g_scratch.push_back({dev, ctx, pool});
+    return pool;
+}
+
+}  // namespace
+
+cudaError_t csg_detail::scratch_alloc(void** p, size_t bytes, cudaStream_t st) {
+    // a captured call takes its memory as before, as nodes of the graph
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(st, &cap) != cudaSuccess) {
+        cudaGetLastError();
+        cap = cudaStreamCaptureStatusActive;
+    }
+    if (cap == cudaStreamCaptureStatusNone) {
+        if (cudaMemPool_t pool = scratch_pool(true)) {
+            if (cudaMallocFromPoolAsync(p, bytes, pool, st) == cudaSuccess) return cudaSuccess;
+            cudaGetLastError();
+        }
+    }
+    return cudaMallocAsync(p, bytes, st);
+}
+
+void csg_detail::scratch_trim() {
+    if (cudaMemPool_t pool = scratch_pool(false))
+        if (cudaMemPoolTrimTo(pool, 0) != cudaSuccess) cudaGetLastError();
+}
+
+namespace {
+
 constexpr int kMaxResidentL = 24;  // largest L of the cluster-resident kernel
 constexpr int kMaxL = 128;         // largest L of the streaming engine
 
@@ -509,7 +591,7 @@ int run_stream(const csg_config& cfg, uint32_t* spins, const uint32_t* bonds,
     CSG_CUDA(cudaGetDevice(&dev));
     CSG_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
     char* base = nullptr;
-    CSG_CUDA(cudaMallocAsync(reinterpret_cast<void**>(&base), lay.bytes, st));
+    CSG_CUDA(scratch_alloc(reinterpret_cast<void**>(&base), lay.bytes, st));
     S.u_acc = reinterpret_cast<int*>(base + lay.u_acc);
     S.up_acc = reinterpret_cast<int*>(base + lay.up_acc);
     S.d_acc = reinterpret_cast<int*>(base + lay.d_acc);
@@ -894,6 +976,7 @@ int csg_engine_destroy(csg_engine* e) {
     if (e->stream) cudaStreamSynchronize(e->stream);
     free_engine(e);
     delete e;
+    scratch_trim();
     return CSG_OK;
 }
 
@@ -1055,7 +1138,7 @@ struct Scratch {
     }
     int take(const csg_engine* e, size_t bytes) {
         const cudaError_t ce = e->pool ? cudaMallocFromPoolAsync(&p, bytes, e->pool, st)
-                                       : cudaMallocAsync(&p, bytes, st);
+                                       : scratch_alloc(&p, bytes, st);
         if (ce == cudaSuccess) return CSG_OK;
         cudaGetLastError();
         p = nullptr;

@@ -75,6 +75,14 @@ CSG_INTERNAL void engine_release(csg_engine* e);
 // Device memory for an engine: from its pool (stream-ordered) or cudaMalloc.
 CSG_INTERNAL int engine_alloc(csg_engine* e, void** p, size_t bytes);
 
+// Scratch of one call, in the order of a stream; give it back with
+// cudaFreeAsync on the same stream.  From a pool of the library's own that
+// keeps up to 64 MB per device between calls (the device's default pool gives its
+// memory back at every synchronisation, and mapping it again costs a call ~400
+// us); scratch_trim gives that back.
+CSG_INTERNAL cudaError_t scratch_alloc(void** p, size_t bytes, cudaStream_t st);
+CSG_INTERNAL void scratch_trim();
+
 // Configuration checks.
 CSG_INTERNAL int validate(const csg_config* cfg);
 CSG_INTERNAL bool use_stream(const csg_config& c);  // streaming engine, not the resident kernel
