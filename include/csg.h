@@ -242,7 +242,7 @@ int csg_obs_records_noalloc(const csg_config* cfg, const uint32_t* spins, const 
  * error (the script's estimators; the error is the standard error over
  * disorder samples).  Runs on stream (NULL: the default stream) and returns
  * when the table is ready; takes ndis * nrep * 72 bytes of stream-ordered
- * scratch. */
+ * scratch, or up to 11 MB where that is less. */
 int csg_analyze_records(const float* rec, int64_t n_meas, int32_t ndis, int32_t nrep, int32_t L,
                         double* table, void* stream);
 
