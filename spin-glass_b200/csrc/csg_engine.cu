@@ -1174,17 +1174,13 @@ int csg_obs_records(csg_engine* e, float* rec, size_t n_floats) {
     const int L = d.L, W = d.n_words, T = d.n_temps;
     const size_t need = (size_t)32 * W * T * 11;
     if (n_floats != need) return fail(CSG_ERR_ARG, "record buffer size mismatch");
-    const size_t nE = (size_t)W * 2 * T * 32, nD = (size_t)W * T * 32, nP = nD * 3 * L;
+    const size_t nE = (size_t)W * 2 * T * 32, nP = (size_t)W * T * 32 * 3 * L;
     // scratch: integers, the phase tables, the records
-    const size_t o_m = nE * 4, o_d = o_m + nE * 4, o_p = o_d + nD * 4, o_cs = (o_p + nP * 4 + 15) & ~(size_t)15;
+    const size_t o_p = 2 * nE * 4, o_cs = (o_p + nP * 4 + 15) & ~(size_t)15;
     const size_t o_rec = o_cs + (size_t)2 * L * 8, bytes = o_rec + need * 4;
     if (!e->rec_scratch)
         if (int rc = engine_alloc(e, reinterpret_cast<void**>(&e->rec_scratch), bytes)) return rc;
     char* sc = e->rec_scratch;
-    int* de = reinterpret_cast<int*>(sc);
-    int* dm = reinterpret_cast<int*>(sc + o_m);
-    int* dd = reinterpret_cast<int*>(sc + o_d);
-    int* dp = reinterpret_cast<int*>(sc + o_p);
     double* dcs = reinterpret_cast<double*>(sc + o_cs);
     float* drec = reinterpret_cast<float*>(sc + o_rec);
     // the L phases exp(i k a), k = 2 pi / L, computed on the host
@@ -1194,20 +1190,10 @@ int csg_obs_records(csg_engine* e, float* rec, size_t n_floats) {
         cs[a] = std::cos(k * a);
         cs[L + a] = std::sin(k * a);
     }
-    // 3L counters per lane; as many warps as fit in 48 KB (4 up to L = 32)
-    const size_t per_warp = (size_t)32 * 3 * L * sizeof(int);
-    const int warps = (int)std::max<size_t>(1, std::min<size_t>(4, 49152 / per_warp));
-    const unsigned blocks = (unsigned)((W * T + warps - 1) / warps);
-    const size_t sh = (size_t)warps * per_warp;
     cudaError_t ce = cudaMemcpyAsync(dcs, cs.data(), cs.size() * 8, cudaMemcpyHostToDevice, e->stream);
-    if (ce == cudaSuccess) {
-        csg::measure_kernel<<<blocks, warps * 32, sh, e->stream>>>(e->spins, e->bonds, L, W, T, de, dm,
-                                                                   dd, dp);
-        const long total = (long)W * 32 * T;
-        csg::records_kernel<<<(unsigned)((total + 127) / 128), 128, 0, e->stream>>>(
-            de, dm, dd, dp, dcs, dcs + L, L, W, T, (float)e->cfg.H, drec);
-        ce = cudaGetLastError();
-    }
+    if (ce == cudaSuccess)
+        ce = csg::records_launch(e->spins, e->bonds, L, W, T, (float)e->cfg.H, reinterpret_cast<int*>(sc),
+                                 reinterpret_cast<int*>(sc + o_p), dcs, dcs + L, drec, e->stream);
     if (ce == cudaSuccess) ce = cudaMemcpyAsync(rec, drec, need * 4, cudaMemcpyDeviceToHost, e->stream);
     if (ce == cudaSuccess) ce = cudaStreamSynchronize(e->stream);
     if (ce != cudaSuccess) return fail(CSG_ERR_CUDA, std::string("records: ") + cudaGetErrorString(ce));

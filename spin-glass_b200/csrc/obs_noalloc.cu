@@ -54,10 +54,11 @@ int csg_obs_records_noalloc(const csg_config* cfg, const uint32_t* spins, const 
     if (d.n_copies != 2) return fail(CSG_ERR_UNSUPPORTED, "observable records need two copies");
     const int L = d.L, W = d.n_words, T = d.n_temps;
     if (n_floats != (size_t)32 * W * T * 11) return fail(CSG_ERR_ARG, "record buffer size mismatch");
-    // scratch layout (ints): e [W][2][T][32], m (same), d [W][T][32],
-    // per-plane d [W][T][32][3L], then the cos/sin table (2L doubles)
+    // scratch layout (ints): unsatisfied bonds [W][2][T][32], spins up (same),
+    // [W][T][32] unused, differing sites per plane [W][T][3L][32], then the
+    // cos/sin table (2L doubles)
     const size_t nE = (size_t)W * 2 * T * 32, nD = (size_t)W * T * 32, nP = nD * 3 * L;
-    const size_t o_m = nE, o_d = 2 * nE, o_p = o_d + nD, o_cs = (o_p + nP + 1) & ~(size_t)1;
+    const size_t o_p = 2 * nE + nD, o_cs = (o_p + nP + 1) & ~(size_t)1;
     const size_t need = o_cs + 4 * (size_t)L;
     if (need > kScratchInts)
         return fail(CSG_ERR_UNSUPPORTED,
@@ -78,32 +79,9 @@ int csg_obs_records_noalloc(const csg_config* cfg, const uint32_t* spins, const 
     cudaError_t e = cudaMemcpyAsync(dcs, cs.data(), cs.size() * sizeof(double),
                                     cudaMemcpyHostToDevice, st);
     if (e != cudaSuccess) return fail(CSG_ERR_CUDA, std::string("table copy: ") + cudaGetErrorString(e));
-    // 3L counters per lane; as many warps as fit in 48 KB (4 up to L = 32)
-    const size_t per_warp = (size_t)32 * 3 * L * sizeof(int);
-    const int warps = (int)std::max<size_t>(1, std::min<size_t>(4, 49152 / per_warp));
-    int* de = scratch;
-    int* dm = scratch + o_m;
-    int* dd = scratch + o_d;
-    int* dp = scratch + o_p;
     // each launch is checked on its own (an error left by the caller's earlier
     // work stays theirs)
-    {
-        void* args[] = {&spins, &bonds, (void*)&L, (void*)&W, (void*)&T, &de, &dm, &dd, &dp};
-        e = cudaLaunchKernel(reinterpret_cast<const void*>(csg::measure_kernel),
-                             dim3((unsigned)((W * T + warps - 1) / warps)), dim3(warps * 32), args,
-                             (size_t)warps * per_warp, st);
-    }
-    if (e != cudaSuccess) return fail(CSG_ERR_CUDA, std::string("launch: ") + cudaGetErrorString(e));
-    {
-        const long total = (long)W * 32 * T;
-        const double* dc = dcs;
-        const double* dsn = dcs + L;
-        const float H = (float)cfg->H;
-        void* args[] = {&de, &dm, &dd, &dp, &dc, &dsn, (void*)&L, (void*)&W, (void*)&T,
-                        (void*)&H, &rec};
-        e = cudaLaunchKernel(reinterpret_cast<const void*>(csg::records_kernel),
-                             dim3((unsigned)((total + 127) / 128)), dim3(128), args, 0, st);
-    }
+    e = csg::records_launch(spins, bonds, L, W, T, (float)cfg->H, scratch, scratch + o_p, dcs, dcs + L, rec, st);
     if (e != cudaSuccess) return fail(CSG_ERR_CUDA, std::string("launch: ") + cudaGetErrorString(e));
     return CSG_OK;
 }

@@ -74,7 +74,7 @@ struct PtParams {
 
 constexpr int kFlagMeasureM = 1;
 
-constexpr int bit_length(int v) {
+__host__ __device__ constexpr int bit_length(int v) {
     int b = 0;
     while (v > 0) {
         ++b;
