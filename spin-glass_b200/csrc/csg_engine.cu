@@ -513,15 +513,17 @@ int colour_planes(const csg::StreamParams& S, int copies, int blocks_per_sm, int
     return best;
 }
 
-using ColourLaunch = void (*)(const csg::StreamParams&, int, int, long long, cudaStream_t);
+using ColourLaunch = void (*)(const csg::StreamParams&, int, int, long long, bool, cudaStream_t);
 
 template <int F, bool E, bool M, int C>
-void launch_colour(const csg::StreamParams& S, int nsm, int p, long long s, cudaStream_t st) {
+void launch_colour(const csg::StreamParams& S, int nsm, int p, long long s, bool back, cudaStream_t st) {
     constexpr int NC = csg::colour_copies<E || M>(C);
     const int zb = colour_planes(S, NC, csg::colour_blocks<F, E, M, NC>(), nsm, E || M);
     const int npb = (S.L * (S.L / 2) + csg::kColourThreads - 1) / csg::kColourThreads;
-    const dim3 grid((unsigned)(S.W * (S.C / NC) * S.Q), (unsigned)(npb * ((S.L + zb - 1) / zb)));
-    launch_pdl(csg::stream_colour_kernel<F, E, M, NC>, grid, dim3(csg::kColourThreads), st, S, p, s, zb);
+    const int chunks = (S.L + zb - 1) / zb;
+    const dim3 grid((unsigned)(S.W * (S.C / NC) * S.Q), (unsigned)(npb * chunks));
+    launch_pdl(csg::stream_colour_kernel<F, E, M, NC>, grid, dim3(csg::kColourThreads), st, S, p, s, zb,
+               back ? (chunks - 1) * zb : 0, back ? -zb : zb);
 }
 
 template <int F, int C>
@@ -611,6 +613,7 @@ int run_stream(const csg_config& cfg, uint32_t* spins, const uint32_t* bonds,
     const dim3 g_overlap(W * Q, (unsigned)lay.nblk2);
     const int64_t sps = cfg.sched.sweeps_per_swap, spm = cfg.sched.sweeps_per_meas;
     cudaError_t ce = cudaSuccess;
+    bool back = false;  // direction of the next pass over the state
     for (int64_t i = 0; i < n_sweeps && ce == cudaSuccess; ++i) {
         const long long s = sweep0 + i;
         const bool do_swap = sps > 0 && (s + 1) % sps == 0;
@@ -621,8 +624,10 @@ int run_stream(const csg_config& cfg, uint32_t* spins, const uint32_t* bonds,
             ce = csg::launch_stream_sweep(S, s, field != csg::kNoField, need_E, need_M, st);
             if (ce != cudaSuccess) break;
         } else {
-            colour_launch(d.n_copies, field, false, need_M)(S, nsm, 0, s, st);
-            colour_launch(d.n_copies, field, need_E, need_M)(S, nsm, 1, s, st);
+            colour_launch(d.n_copies, field, false, need_M)(S, nsm, 0, s, back, st);
+            back = !back;
+            colour_launch(d.n_copies, field, need_E, need_M)(S, nsm, 1, s, back, st);
+            back = !back;
         }
         if (need_E) {
             const long long round = do_swap ? (s + 1) / sps - 1 : 0;
@@ -632,12 +637,14 @@ int run_stream(const csg_config& cfg, uint32_t* spins, const uint32_t* bonds,
                        log_rounds);
             const bool overlap = do_meas && obs && C == 2;
             if (do_swap && overlap)  // one pass: exchange, then count the overlaps
-                launch_pdl(csg::stream_exchange_overlap_kernel, dim3(W, (unsigned)lay.nblk2),
-                           dim3(csg::kStreamThreads), st, S, par);
+                launch_pdl(csg::stream_exchange_overlap_kernel,
+                           dim3(W, (unsigned)((N + csg::kExchangeSitesPerBlock - 1) / csg::kExchangeSitesPerBlock)),
+                           dim3(csg::kStreamThreads), st, S, par, back);
             else if (do_swap)
-                launch_pdl(csg::stream_exchange_kernel, g_exchange, dim3(256), st, S, par);
+                launch_pdl(csg::stream_exchange_kernel, g_exchange, dim3(256), st, S, par, back);
             else if (overlap)
                 launch_pdl(csg::stream_overlap_kernel, g_overlap, dim3(csg::kStreamThreads), st, S);
+            if (do_swap) back = !back;
             if (do_meas && obs)
                 launch_pdl(csg::stream_measure_kernel, dim3(W * (unsigned)d.n_temps), dim3(64), st, S,
                            need_M, O);

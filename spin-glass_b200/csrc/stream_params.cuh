@@ -37,6 +37,14 @@ constexpr int kOverlapSPT = 8;
 constexpr int kOverlapSitesPerBlock = kStreamThreads * kOverlapSPT;
 constexpr int kOverlapNL = bit_length(kOverlapSPT);
 
+// Exchange and overlap pass: sites per thread.  Two leave 64 registers and
+// blocks of 512 sites (4 blocks an SM, 512 blocks at L = 32 and 256 samples,
+// where blocks of 2048 were 128 for 148 SMs); four: 119 registers, 1 to 5 %
+// slower a pass of the engine.
+constexpr int kExchangeSites = 2;
+constexpr int kExchangeSitesPerBlock = kStreamThreads * kExchangeSites;
+constexpr int kExchangeNL = bit_length(kExchangeSites);
+
 struct StreamParams {
     uint32_t* spins;
     const uint32_t* bonds;
