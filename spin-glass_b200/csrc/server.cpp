@@ -23,22 +23,6 @@
 
 using namespace csg_detail;
 
-namespace {
-
-// Plan for a request that shares the GPU with others: the largest split of
-// quads that fits one CTA with the default column split (fewest CTAs and
-// cluster barriers per unit of work); automatic (the single-request plan) for
-// the streaming engine.
-PlanChoice shared_gpu_plan(const csg_config& c) {
-    const std::vector<PlanChoice> opts = plan_options(c, true);
-    PlanChoice best{};
-    for (const PlanChoice& o : opts)
-        if (o.nseg == opts.front().nseg && o.qc > best.qc) best = o;
-    return best;
-}
-
-}  // namespace
-
 struct csg_server {
     struct Req {
         int64_t id;
@@ -227,13 +211,24 @@ int csg_server_poll(csg_server* s, int64_t* completed, int32_t max_completed,
             --running;
         }
     }
+    // alone, a request takes the plan that spreads it widest; sharing the GPU,
+    // the tiles shared_plans finds for all that run (every plan gives the same
+    // bits)
+    std::vector<SharedLoad> loads;
+    std::vector<const csg_server::Req*> of;
+    std::vector<PlanChoice> plans;
+    for (const auto& r : s->active)
+        if (!r.done) {
+            loads.push_back({&r.cfg, r.total - r.launched});
+            of.push_back(&r);
+        }
     for (auto& r : s->active) {
         if (r.done || r.launched >= r.total) continue;
         if (cudaStreamQuery(r.stream) != cudaSuccess) continue;
+        if (running > 1 && plans.empty()) plans = shared_plans(loads);
         const int64_t n = std::min<int64_t>(s->chunk, r.total - r.launched);
-        // alone, a request takes the plan that spreads it widest; sharing the
-        // GPU, the one with the fewest CTAs (every plan gives the same bits)
-        const PlanChoice pc = running > 1 ? shared_gpu_plan(r.cfg) : PlanChoice{};
+        const size_t k = (size_t)(std::find(of.begin(), of.end(), &r) - of.begin());
+        const PlanChoice pc = running > 1 && k < plans.size() ? plans[k] : PlanChoice{};
         r.e->qc = pc.qc;
         r.e->nseg = pc.nseg;
         if (int rc = csg_run(r.e, n)) {
