@@ -45,18 +45,28 @@ static __global__ void init_kernel(uint32_t* spins, uint32_t* bonds, int L, int 
         }
 }
 
+// The 4 planes of a quad at site n: one load, or four where the caller's spins
+// are not on a 16-byte boundary (csg_obs_records_noalloc takes any).
+template <bool ALIGNED>
+__device__ __forceinline__ uint4 quad_at(const uint32_t* quad, int n) {
+    if constexpr (ALIGNED) return reinterpret_cast<const uint4*>(quad)[n];
+    const uint32_t* p = quad + (size_t)4 * n;
+    return make_uint4(p[0], p[1], p[2], p[3]);
+}
+
 constexpr int kCountThreads = 256;
 constexpr int kCountSites = 16;  // sites per thread of the bond counts
 
 // Unsatisfied bonds u[w][c][t][b] and spins up n_up[w][c][t][b], added to what is
 // there: blockIdx.x = quad (w, c, q), blockIdx.y = part of the sites (at most
 // kCountSites per thread).
+template <bool ALIGNED>
 static __global__ void __launch_bounds__(kCountThreads) bond_counts_kernel(
     const uint32_t* __restrict__ spins, const uint32_t* __restrict__ bonds, int L, int T, int* u, int* n_up) {
     constexpr int NLU = bit_length(3 * kCountSites), NLM = bit_length(kCountSites);
     const int LH = L / 2, PL = L * LH, NH = L * PL, N = 2 * NH, Q = T / 4;
     const int gq = blockIdx.x, w = gq / (2 * Q), lane = threadIdx.x & 31;
-    const uint4* const S = reinterpret_cast<const uint4*>(spins) + (size_t)gq * N;
+    const uint32_t* const S = spins + (size_t)gq * N * 4;
     const uint32_t* const F = bonds + (size_t)w * 3 * N;
     __shared__ int sum[2][4][32];
     (&sum[0][0][0])[threadIdx.x] = 0;
@@ -71,11 +81,11 @@ static __global__ void __launch_bounds__(kCountThreads) bond_counts_kernel(
         const int z = (int)(((float)m + 0.5f) * inv_pl), r = m - z * PL;
         const int y = (int)(((float)r + 0.5f) * inv_lh), h = r - y * LH;
         const int o = (y + z + p) & 1;  // x = 2h + o
-        const uint4* const So = S + (1 - p) * NH + m;
-        const uint4 s = S[n];
-        const uint4 ax = So[o ? (h == LH - 1 ? 1 - LH : 1) : 0];
-        const uint4 ay = So[y == L - 1 ? LH - PL : LH];
-        const uint4 az = So[z == L - 1 ? PL - NH : PL];
+        const int no = (1 - p) * NH + m;
+        const uint4 s = quad_at<ALIGNED>(S, n);
+        const uint4 ax = quad_at<ALIGNED>(S, no + (o ? (h == LH - 1 ? 1 - LH : 1) : 0));
+        const uint4 ay = quad_at<ALIGNED>(S, no + (y == L - 1 ? LH - PL : LH));
+        const uint4 az = quad_at<ALIGNED>(S, no + (z == L - 1 ? PL - NH : PL));
         const uint32_t fx = F[n], fy = F[N + n], fz = F[2 * N + n];
         const uint32_t sw[4] = {s.x, s.y, s.z, s.w}, xw[4] = {ax.x, ax.y, ax.z, ax.w};
         const uint32_t yw[4] = {ay.x, ay.y, ay.z, ay.w}, zw[4] = {az.x, az.y, az.z, az.w};
@@ -117,7 +127,7 @@ static __global__ void __launch_bounds__(kCountThreads) bond_counts_kernel(
 // Sites where the copies differ in each coordinate plane, diff[w][t][dir][a][b]
 // (dir 0, 1, 2 = x, y, z equal to a): a warp per (w, q, dir, a), blockIdx.x = (w,
 // q), blockIdx.y = 4 of the 3L planes.  NL: bits of a lane's count, L L / 32 sites.
-template <int NL>
+template <int NL, bool ALIGNED>
 static __global__ void __launch_bounds__(128) overlap_planes_kernel(const uint32_t* __restrict__ spins, int L, int T,
                                                                     int* __restrict__ diff) {
     const int LH = L / 2, PL = L * LH, NH = L * PL, N = 2 * NH, Q = T / 4;
@@ -125,8 +135,8 @@ static __global__ void __launch_bounds__(128) overlap_planes_kernel(const uint32
     const int plane = blockIdx.y * 4 + (threadIdx.x >> 5);
     if (plane >= 3 * L) return;
     const int dir = plane / L, a = plane - dir * L;
-    const uint4* const A = reinterpret_cast<const uint4*>(spins) + ((size_t)(w * 2) * Q + q) * N;
-    const uint4* const B = A + (size_t)Q * N;
+    const uint32_t* const A = spins + ((size_t)(w * 2) * Q + q) * N * 4;
+    const uint32_t* const B = A + (size_t)Q * N * 4;
     uint32_t cd[4][NL] = {};
     const float inv_l = 1.0f / (float)L, inv_lh = 1.0f / (float)LH;
     for (int i = lane; i < L * L; i += 32) {
@@ -140,7 +150,7 @@ static __global__ void __launch_bounds__(128) overlap_planes_kernel(const uint32
             const int z = (int)(((float)i + 0.5f) * inv_l), y = i - z * L;
             n = ((a + y + z) & 1) * NH + i * LH + (a >> 1);
         }
-        const uint4 v = A[n], x = B[n];
+        const uint4 v = quad_at<ALIGNED>(A, n), x = quad_at<ALIGNED>(B, n);
         const uint32_t d[4] = {v.x ^ x.x, v.y ^ x.y, v.z ^ x.z, v.w ^ x.w};
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
@@ -198,6 +208,15 @@ static __global__ void records_kernel(const int* __restrict__ u, const int* __re
     o[4] = (float)(N - 2 * D) / (float)N;
 }
 
+template <bool ALIGNED>
+static const void* overlap_planes_for(int L) {
+    const int sites = (L * L + 31) / 32;  // of a plane per lane
+    return sites <= 3    ? reinterpret_cast<const void*>(overlap_planes_kernel<2, ALIGNED>)
+           : sites <= 15 ? reinterpret_cast<const void*>(overlap_planes_kernel<4, ALIGNED>)
+           : sites <= 63 ? reinterpret_cast<const void*>(overlap_planes_kernel<6, ALIGNED>)
+                         : reinterpret_cast<const void*>(overlap_planes_kernel<10, ALIGNED>);
+}
+
 // Queues the records of a state on a stream.  counts: 2 W 2 T 32 ints (unsatisfied
 // bonds, then spins up); diff: W T 32 3L ints; all of them written before they are
 // read.  Bound: the loads, a pass over the spins and their neighbours and three
@@ -209,6 +228,7 @@ static inline cudaError_t records_launch(const uint32_t* spins, const uint32_t* 
     const size_t n_e = (size_t)W * 2 * T * 32;
     const int Q = T / 4;
     const long N = (long)L * L * L;
+    const bool aligned = reinterpret_cast<uintptr_t>(spins) % 16 == 0;
     int* u = counts;
     int* n_up = counts + n_e;
     cudaError_t ce = cudaMemsetAsync(counts, 0, 2 * n_e * sizeof(int), st);
@@ -216,19 +236,16 @@ static inline cudaError_t records_launch(const uint32_t* spins, const uint32_t* 
     {
         const long per_block = (long)kCountThreads * kCountSites;
         void* args[] = {&spins, &bonds, &L, &T, &u, &n_up};
-        ce = cudaLaunchKernel(reinterpret_cast<const void*>(bond_counts_kernel),
+        ce = cudaLaunchKernel(aligned ? reinterpret_cast<const void*>(bond_counts_kernel<true>)
+                                      : reinterpret_cast<const void*>(bond_counts_kernel<false>),
                               dim3((unsigned)(W * 2 * Q), (unsigned)((N + per_block - 1) / per_block)),
                               dim3(kCountThreads), args, 0, st);
         if (ce != cudaSuccess) return ce;
     }
     {
-        const int sites = (L * L + 31) / 32;  // of a plane per lane
-        const void* fn = sites <= 3    ? reinterpret_cast<const void*>(overlap_planes_kernel<2>)
-                         : sites <= 15 ? reinterpret_cast<const void*>(overlap_planes_kernel<4>)
-                         : sites <= 63 ? reinterpret_cast<const void*>(overlap_planes_kernel<6>)
-                                       : reinterpret_cast<const void*>(overlap_planes_kernel<10>);
         void* args[] = {&spins, &L, &T, &diff};
-        ce = cudaLaunchKernel(fn, dim3((unsigned)(W * Q), (unsigned)((3 * L + 3) / 4)), dim3(128), args, 0, st);
+        ce = cudaLaunchKernel(aligned ? overlap_planes_for<true>(L) : overlap_planes_for<false>(L),
+                              dim3((unsigned)(W * Q), (unsigned)((3 * L + 3) / 4)), dim3(128), args, 0, st);
         if (ce != cudaSuccess) return ce;
     }
     const long total = (long)W * 32 * T;

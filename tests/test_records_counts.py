@@ -41,3 +41,29 @@ def test_records_of_a_random_state(csg, L, W, T):
                     f = (q.sum(axis=tuple(i for i in range(3) if i != 2 - k)) * wave).sum() / N
                     want[5 + k], want[8 + k] = f.real, f.imag
                 np.testing.assert_allclose(rec[32 * w + b, t], want, atol=1e-6, err_msg=f"{w} {b} {t}")
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("L", [6, 12, 22])
+def test_records_of_spins_off_a_16_byte_boundary(csg, L):
+    """csg_obs_records_noalloc takes spins at any 4-byte address."""
+    import ctypes as C
+    import torch
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    f = csg.lib().csg_obs_records_noalloc
+    f.argtypes = [C.POINTER(csg.Config), C.c_void_p, C.c_void_p, C.c_void_p, C.c_size_t, C.c_void_p]
+    W, T = 1, 8
+    with csg.Engine(L, W, 2, np.linspace(2.0, 0.5, T), seed=3) as e:
+        e.init_lattice()
+        want = e.obs_records()
+        s, b, _ = e.get_state()
+        db = torch.from_numpy(b.view(np.int32).reshape(-1)).cuda()
+        for off in (0, 1, 2, 3):
+            ds = torch.zeros(s.size + 4, dtype=torch.int32, device="cuda")
+            ds[off:off + s.size] = torch.from_numpy(s.view(np.int32).reshape(-1))
+            out = torch.zeros((32 * W, T, 11), device="cuda")
+            assert f(C.byref(e.cfg), ds.data_ptr() + 4 * off, db.data_ptr(), out.data_ptr(), out.numel(),
+                     torch.cuda.current_stream().cuda_stream) == 0
+            torch.cuda.synchronize()
+            np.testing.assert_array_equal(out.cpu().numpy(), want)
