@@ -217,7 +217,10 @@ __global__ void __launch_bounds__(max_cta_threads(FIELD != kNoField, NSEG)) pt_r
         const uint32_t s32 = (uint32_t)s;
         const PhiloxFixed pf = philox_fix(s32, wg, ctr3, P.k0, P.k1);
 
+        // the loops from here on run once or a few times: unrolled they only cost
+        // instruction cache and the site loop's registers
         if (need_E)  // sE, sD and (if present) sM are contiguous
+#pragma unroll 1
             for (int i = tid; i < Qc * 4 * 32 * (has_M ? 3 : 2); i += nthreads) sE[i] = 0;
 
         BondCounts<NLV> ecnt[4];
@@ -399,6 +402,7 @@ __global__ void __launch_bounds__(max_cta_threads(FIELD != kNoField, NSEG)) pt_r
             // CTA of the cluster).
             if (par) cluster.sync();
             else __syncthreads();
+#pragma unroll 1
             for (int pi = warp; pi < 2 * Qc; pi += nwarps) {
                 const int jj = pi >> 1;
                 const int tq = par + 2 * (pi & 1);
@@ -474,6 +478,7 @@ __global__ void __launch_bounds__(max_cta_threads(FIELD != kNoField, NSEG)) pt_r
                     x ^= d;
                     y ^= d;
                 };
+#pragma unroll 1
                 for (int i0 = lt; i0 < N4; i0 += CH * TPQ) {
                     uint4 a[CH], b[CH];
 #pragma unroll
@@ -520,22 +525,32 @@ __global__ void __launch_bounds__(max_cta_threads(FIELD != kNoField, NSEG)) pt_r
         }
 
         if (do_meas) {
-            for (int i = tid; i < Qc * 4 * 32; i += nthreads) {
-                const int pl = i >> 5, b = i & 31;
-                const int gg = rank * Qc + (pl >> 2);
-                const int cc = gg % C, t = 4 * (gg / C) + (pl & 3);
-                const size_t o = (((size_t)w * C + cc) * T + t) * 32 + b;
-                const int ev = 2 * sE[i] - 3 * N;
-                if (P.e_sum) atomicAdd(reinterpret_cast<unsigned long long*>(P.e_sum + o),
-                                       (unsigned long long)(long long)ev);
-                if (P.e_last) P.e_last[o] = ev;
-                if (need_M) {
-                    const int mv = 2 * sM[i] - N;
-                    if (P.m_sum) atomicAdd(reinterpret_cast<unsigned long long*>(P.m_sum + o),
-                                           (unsigned long long)(long long)mv);
-                    if (P.m_last) P.m_last[o] = mv;
+            // Global atomics: last in the sweep they have the next one to land
+            // in, where right before a cluster barrier that barrier waits for them
+            // (production shape 24.5 -> 24.1 us a sweep).  Large teams of short
+            // columns hide them behind the overlap counts instead (one word at L
+            // = 12, 288 threads a quad: 8.2 us last, 8.1 first).
+            constexpr bool kEnergiesLast = ZS >= 4;
+            auto add_energies = [&] {
+#pragma unroll 1
+                for (int i = tid; i < Qc * 4 * 32; i += nthreads) {
+                    const int pl = i >> 5, b = i & 31;
+                    const int gg = rank * Qc + (pl >> 2);
+                    const int cc = gg % C, t = 4 * (gg / C) + (pl & 3);
+                    const size_t o = (((size_t)w * C + cc) * T + t) * 32 + b;
+                    const int ev = 2 * sE[i] - 3 * N;
+                    if (P.e_sum) atomicAdd(reinterpret_cast<unsigned long long*>(P.e_sum + o),
+                                           (unsigned long long)(long long)ev);
+                    if (P.e_last) P.e_last[o] = ev;
+                    if (need_M) {
+                        const int mv = 2 * sM[i] - N;
+                        if (P.m_sum) atomicAdd(reinterpret_cast<unsigned long long*>(P.m_sum + o),
+                                               (unsigned long long)(long long)mv);
+                        if (P.m_last) P.m_last[o] = mv;
+                    }
                 }
-            }
+            };
+            if constexpr (!kEnergiesLast) add_energies();
             if (C == 2) {
                 if (!do_swap) cluster.sync();  // partner copies finished the sweep
                 // Overlap of quad q: the copy-0 team counts the colour-0 sites,
@@ -572,6 +587,7 @@ __global__ void __launch_bounds__(max_cta_threads(FIELD != kNoField, NSEG)) pt_r
                     return r0 == rank ? sD + j0 * 4 * 32 : cluster.map_shared_rank(sD + j0 * 4 * 32, r0);
                 });
                 cluster.sync();  // all counts in; partner planes may be modified again
+#pragma unroll 1
                 for (int i = tid; i < Qc * 4 * 32; i += nthreads) {
                     const int pl = i >> 5, b = i & 31;
                     const int gg = rank * Qc + (pl >> 2);
@@ -595,6 +611,7 @@ __global__ void __launch_bounds__(max_cta_threads(FIELD != kNoField, NSEG)) pt_r
                     if (P.d_last) P.d_last[o] = D;
                 }
             }
+            if constexpr (kEnergiesLast) add_energies();
             __syncthreads();  // sE / sD are cleared at the start of the next sweep
         }
     }
