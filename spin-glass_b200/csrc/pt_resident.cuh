@@ -5,8 +5,8 @@
 //     (Walk<L, NSEG>): for every site it loads the 4 temperature planes of the
 //     site and its six neighbours from shared memory at offsets fixed for the
 //     launch, draws one Philox block for the 4 planes, counts unsatisfied
-//     bonds with two full adders per triple and takes the flip mask from the
-//     threshold table.
+//     bonds with two full adders per triple and forms the flip mask from
+//     them and the masks of the draw against the thresholds (pt_kernel.cuh).
 //   energies — while colour 1 runs, the post-flip unsatisfied-bond counts are
 //     added into bit-sliced per-thread counters (each bond has exactly one
 //     colour-1 end); warps reduce them with a 32x32 bit transpose + popc.
