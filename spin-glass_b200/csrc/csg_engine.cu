@@ -1217,6 +1217,10 @@ struct Scratch {
     }
 };
 
+int checkpoint_failed(cudaError_t ce) {
+    return fail(CSG_ERR_CUDA, std::string("checkpoint: ") + cudaGetErrorString(ce));
+}
+
 // Scratch for the checkpoint of `words` words of samples at once (and extra
 // bytes): all of them up to 256 MB, fewer where the device cannot hold that.
 constexpr size_t kCheckpointScratch = (size_t)256 << 20;
@@ -1286,16 +1290,20 @@ int csg_save_checkpoint(csg_engine* e, uint32_t* ref, size_t n_words) {
     Scratch sc(e->stream);
     if (int rc = checkpoint_scratch(e, sc, step, 0)) return rc;
     uint32_t* dev = static_cast<uint32_t*>(sc.p);
-    for (int w0 = 0; w0 < W; w0 += step) {
+    cudaError_t ce = cudaSuccess;
+    for (int w0 = 0; w0 < W && ce == cudaSuccess; w0 += step) {
         const int n = std::min(step, W - w0);
         csg::checkpoint_save_kernel<<<dim3((unsigned)((N + 127) / 128), (unsigned)(2 * n)), 128, 0, e->stream>>>(
             e->spins, e->bonds, csg::CheckpointDims{L, T, w0, n}, dev);
-        CSG_CUDA(cudaGetLastError());
-        CSG_CUDA(cudaMemcpyAsync(ref + (size_t)64 * w0 * N, dev, (size_t)64 * n * N * 4, cudaMemcpyDeviceToHost,
-                                 e->stream));
+        ce = cudaGetLastError();
+        if (ce == cudaSuccess)
+            ce = cudaMemcpyAsync(ref + (size_t)64 * w0 * N, dev, (size_t)64 * n * N * 4, cudaMemcpyDeviceToHost,
+                                 e->stream);
     }
-    CSG_CUDA(cudaStreamSynchronize(e->stream));
-    return CSG_OK;
+    // ref is the caller's again when this returns, with an error too
+    const cudaError_t done = cudaStreamSynchronize(e->stream);
+    if (ce == cudaSuccess) ce = done;
+    return ce == cudaSuccess ? CSG_OK : checkpoint_failed(ce);
 }
 
 int csg_load_checkpoint(csg_engine* e, const uint32_t* ref, size_t n_words, int64_t sweep) {
@@ -1318,27 +1326,38 @@ int csg_load_checkpoint(csg_engine* e, const uint32_t* ref, size_t n_words, int6
                                e->stream);
     };
     // check all of it before the engine's state is touched
-    CSG_CUDA(cudaMemsetAsync(first, 0xFF, 8, e->stream));
-    for (int w0 = 0; w0 < W; w0 += step) {
+    unsigned long long bad = 0;
+    cudaError_t ce = cudaMemsetAsync(first, 0xFF, 8, e->stream);
+    for (int w0 = 0; w0 < W && ce == cudaSuccess; w0 += step) {
         const int n = std::min(step, W - w0);
-        CSG_CUDA(upload(w0, n));
+        ce = upload(w0, n);
+        if (ce != cudaSuccess) break;
         csg::checkpoint_check_kernel<<<dim3(nb, (unsigned)n), 128, 0, e->stream>>>(
             dev, csg::CheckpointDims{L, T, w0, n}, first);
-        CSG_CUDA(cudaGetLastError());
+        ce = cudaGetLastError();
     }
-    unsigned long long bad = 0;
-    CSG_CUDA(cudaMemcpyAsync(&bad, first, 8, cudaMemcpyDeviceToHost, e->stream));
-    CSG_CUDA(cudaStreamSynchronize(e->stream));
+    if (ce == cudaSuccess) ce = cudaMemcpyAsync(&bad, first, 8, cudaMemcpyDeviceToHost, e->stream);
+    // ref is the caller's again when this returns, with an error too: a copy from
+    // page-locked memory runs on after the call that queued it
+    cudaError_t done = cudaStreamSynchronize(e->stream);
+    if (ce == cudaSuccess) ce = done;
+    if (ce != cudaSuccess) return checkpoint_failed(ce);
     if (bad != ~0ull)
         return fail(CSG_ERR_STATE, bad & 1 ? "the two ends of a bond disagree" : "copies of a sample disagree on its bonds");
     if (sweep < 0) return fail(CSG_ERR_ARG, "negative sweep index");
-    for (int w0 = 0; w0 < W; w0 += step) {
+    for (int w0 = 0; w0 < W && ce == cudaSuccess; w0 += step) {
         const int n = std::min(step, W - w0);
-        if (step < W) CSG_CUDA(upload(w0, n));  // else it is still there
+        if (step < W) ce = upload(w0, n);  // else it is still there
+        if (ce != cudaSuccess) break;
         csg::checkpoint_load_kernel<<<dim3(nb, (unsigned)(2 * n)), 128, 0, e->stream>>>(
             dev, csg::CheckpointDims{L, T, w0, n}, e->spins, e->bonds);
-        CSG_CUDA(cudaGetLastError());
+        ce = cudaGetLastError();
     }
+    if (step < W) {
+        done = cudaStreamSynchronize(e->stream);
+        if (ce == cudaSuccess) ce = done;
+    }
+    if (ce != cudaSuccess) return checkpoint_failed(ce);
     e->sweep = sweep;
     return reset_obs(e);
 }

@@ -1,0 +1,84 @@
+"""The library's host side against a stand-in for the CUDA runtime
+(fake_cudart.cpp), on a machine without a GPU: what a call has finished with
+when it returns, and what it does where the device refuses something."""
+import ctypes as C
+import importlib.util
+import pathlib
+import subprocess
+import sys
+
+import numpy as np
+import pytest
+
+ROOT = pathlib.Path(__file__).resolve().parents[1]
+PKG = ROOT / "spin-glass_b200"
+
+
+def _module(name, path):
+    spec = importlib.util.spec_from_file_location(name, path)
+    mod = importlib.util.module_from_spec(spec)
+    spec.loader.exec_module(mod)
+    return mod
+
+
+@pytest.fixture(scope="module")
+def host(tmp_path_factory):
+    """The package bound to the library's objects linked with the stand-in."""
+    build = _module("csg_build", PKG / "build.py")
+    missing = [u for u in build._units() if not u[0].exists()]
+    build.build_lib(force=bool(missing))
+    so = tmp_path_factory.mktemp("fake") / "libcsg_fake.so"
+    cuda = pathlib.Path(build.NVCC).resolve().parent.parent if "/" in build.NVCC else pathlib.Path("/usr/local/cuda")
+    subprocess.run(["g++", "-shared", "-fPIC", "-O1", "-std=c++17", f"-I{cuda / 'include'}", "-Wl,-Bsymbolic",
+                    str(ROOT / "tests" / "fake_cudart.cpp"), *[str(o) for o, _ in build._units()], "-o", str(so)],
+                   check=True)
+    mod = _module("spin_glass_b200_host", PKG / "__init__.py")
+    mod.LIB_PATH = so
+    L = mod.lib()
+    for name, args, res in (("fake_limit", [C.c_size_t], None), ("fake_max_cluster", [C.c_int], None),
+                            ("fake_refuse_launch", [C.c_int], None),
+                            ("fake_kept", [], C.c_size_t), ("fake_pending", [C.c_void_p, C.c_size_t], C.c_size_t)):
+        f = getattr(L, name)
+        f.argtypes, f.restype = args, res
+    return mod
+
+
+@pytest.fixture
+def fake(host):
+    L = host.lib()
+    yield L
+    L.fake_limit(C.c_size_t(-1).value)
+    L.fake_max_cluster(16)
+    L.fake_refuse_launch(-1)
+
+
+BETAS = np.linspace(2.0, 0.5, 8)
+
+
+@pytest.mark.parametrize("words", [1, 2, 3])
+def test_checkpoint_calls_are_done_with_the_callers_memory(host, fake, words):
+    # room for `words` words of the checkpoint at once: 3, 2 and 1 uploads each way
+    L, W = 4, 3
+    ref = np.zeros((64 * W, L ** 3), np.uint32)
+    with host.Engine(L, W, 2, BETAS, seed=1) as e:
+        fake.fake_limit(words * 64 * L ** 3 * 4 + 8)
+        e.load_checkpoint(ref, 0)
+        assert fake.fake_pending(ref.ctypes.data, ref.nbytes) == 0
+        host._check(fake.csg_save_checkpoint(e._h, host._p(ref), ref.size))
+        assert fake.fake_pending(ref.ctypes.data, ref.nbytes) == 0
+
+
+@pytest.mark.parametrize("call,launch", [("save", 1), ("load", 1), ("load", 3), ("load", 5)])
+def test_checkpoint_calls_that_fail_are_done_with_the_callers_memory(host, fake, call, launch):
+    # a launch is refused after copies of other words were queued
+    L, W = 4, 3
+    ref = np.zeros((64 * W, L ** 3), np.uint32)
+    with host.Engine(L, W, 2, BETAS, seed=1) as e:
+        fake.fake_limit(64 * L ** 3 * 4 + 8)
+        fake.fake_refuse_launch(launch)
+        with pytest.raises(host.CsgError):
+            if call == "load":
+                e.load_checkpoint(ref, 0)
+            else:
+                host._check(fake.csg_save_checkpoint(e._h, host._p(ref), ref.size))
+        assert fake.fake_pending(ref.ctypes.data, ref.nbytes) == 0
