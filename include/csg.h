@@ -195,9 +195,18 @@ int csg_load_checkpoint(csg_engine* e, const uint32_t* ref, size_t n_words, int6
  * (may be NULL).  stream: a cudaStream_t (NULL = legacy default stream).
  * Queued on the stream; the cluster-resident kernel (L <= 24) allocates
  * nothing, the streaming engine (L > 24 or CSG_ENGINE_STREAM) takes a few MB
- * of stream-ordered scratch (cudaMallocAsync / cudaFreeAsync on the stream). */
+ * of scratch in the order of the stream (see csg_trim_scratch; while the stream
+ * is captured, from the device's default pool, as nodes of the graph). */
 int csg_pt_run_device(const csg_config* cfg, uint32_t* spins, const uint32_t* bonds,
                       const csg_device_obs* obs, int64_t sweep0, int64_t n_sweeps, void* stream);
+
+/* No counterpart in the reference.  Scratch of the streaming engine, of
+ * checkpoints and of csg_analyze_records comes from a memory pool of the
+ * library's own, which keeps up to 64 MiB per device between calls.  Destroying an
+ * engine, a batch or a server gives what is kept unused on the current device
+ * back to it, and so does this call, for callers who hold none of them.  Scratch
+ * of work that is still queued stays: wait for the stream first. */
+int csg_trim_scratch(void);
 
 /* init_multispins + init_coupling_constants (eamsim.cu:562-619) into
  * caller-owned device buffers, from the seed. */
@@ -241,8 +250,8 @@ int csg_obs_records_noalloc(const csg_config* cfg, const uint32_t* spins, const 
  * [nrep][8] receiving chi_0, its error, xi_L/L, its error, e, its error, m, its
  * error (the script's estimators; the error is the standard error over
  * disorder samples).  Runs on stream (NULL: the default stream) and returns
- * when the table is ready; takes ndis * nrep * 72 bytes of stream-ordered
- * scratch, or up to 11 MB where that is less. */
+ * when the table is ready; takes ndis * nrep * 72 bytes of scratch in the order
+ * of the stream (csg_trim_scratch), or up to 11 MB where that is less. */
 int csg_analyze_records(const float* rec, int64_t n_meas, int32_t ndis, int32_t nrep, int32_t L,
                         double* table, void* stream);
 

@@ -99,6 +99,7 @@ def lib():
             "csg_load_checkpoint": [vp, vp, sz, i64],
             "csg_pt_run_device": [pcfg, vp, vp, C.POINTER(DeviceObs), i64, i64, vp],
             "csg_init_device": [pcfg, vp, vp, vp],
+            "csg_trim_scratch": [],
             "csg_query_plan": [pcfg, C.POINTER(Plan)],
             "csg_set_plan_override": [C.POINTER(Plan)],
             "csg_batch_create": [C.POINTER(Config), C.c_int32, C.POINTER(vp)],
@@ -301,6 +302,11 @@ def run_device(cfg: Config, spins_ptr: int, bonds_ptr: int, obs: DeviceObs | Non
 def init_device(cfg: Config, spins_ptr: int, bonds_ptr: int, stream: int = 0) -> None:
     _check(lib().csg_init_device(C.byref(cfg), C.c_void_p(spins_ptr), C.c_void_p(bonds_ptr),
                                  C.c_void_p(stream) if stream else None))
+
+
+def trim_scratch() -> None:
+    """Give the scratch the library keeps unused back to the current device."""
+    _check(lib().csg_trim_scratch())
 
 
 def geometric_betas(T: int, t_min: float, t_max: float) -> np.ndarray:

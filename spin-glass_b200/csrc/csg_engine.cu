@@ -944,8 +944,15 @@ int reset_obs(csg_engine* e) {
 int csg_detail::engine_alloc(csg_engine* e, void** p, size_t bytes) {
     *p = nullptr;
     if (bytes == 0) return CSG_OK;
-    const cudaError_t ce = e->pool ? cudaMallocFromPoolAsync(p, bytes, e->pool, e->stream)
-                                   : cudaMalloc(p, bytes);
+    auto take = [&] {
+        return e->pool ? cudaMallocFromPoolAsync(p, bytes, e->pool, e->stream) : cudaMalloc(p, bytes);
+    };
+    cudaError_t ce = take();
+    if (ce == cudaErrorMemoryAllocation) {  // perhaps for the scratch kept between calls
+        cudaGetLastError();
+        scratch_trim();
+        ce = take();
+    }
     if (ce != cudaSuccess) {
         cudaGetLastError();
         *p = nullptr;
@@ -1047,6 +1054,11 @@ int csg_engine_destroy(csg_engine* e) {
     if (e->stream) cudaStreamSynchronize(e->stream);
     free_engine(e);
     delete e;
+    scratch_trim();
+    return CSG_OK;
+}
+
+int csg_trim_scratch(void) {
     scratch_trim();
     return CSG_OK;
 }

@@ -77,9 +77,11 @@ CSG_INTERNAL int engine_alloc(csg_engine* e, void** p, size_t bytes);
 
 // Scratch of one call, in the order of a stream; give it back with
 // cudaFreeAsync on the same stream.  From a pool of the library's own that
-// keeps up to 64 MB per device between calls (the device's default pool gives its
-// memory back at every synchronisation, and mapping it again costs a call ~400
-// us); scratch_trim gives that back.
+// keeps up to 64 MiB per device context between calls (the device's default
+// pool gives its memory back at every synchronisation, and mapping it again
+// costs a call ~400 us); scratch_trim gives back what the current context's
+// pool keeps unused (destroying an engine, a batch or a server does, and
+// csg_trim_scratch).
 CSG_INTERNAL cudaError_t scratch_alloc(void** p, size_t bytes, cudaStream_t st);
 CSG_INTERNAL void scratch_trim();
 

@@ -105,6 +105,7 @@ void destroy_server(csg_server* s) {
     }
     if (s->pool) cudaMemPoolDestroy(s->pool);
     delete s;
+    scratch_trim();  // streamed requests take their scratch from the library's pool
 }
 
 }  // namespace

@@ -35,7 +35,7 @@ std::map<void*, Block> g_blocks;
 std::vector<Stream*> g_streams;
 std::vector<Pool*> g_pools;
 Stream g_default;
-size_t g_limit = SIZE_MAX;
+size_t g_limit = SIZE_MAX, g_capacity = SIZE_MAX;
 int g_max_cluster = 16;
 int g_launches_to_error = -1;
 bool g_error = false;
@@ -70,7 +70,11 @@ void drain_all() {
 
 int take(void** p, size_t n, Pool* pool) {
     *p = nullptr;
-    if (n > g_limit) return cudaErrorMemoryAllocation;
+    size_t held = 0;
+    for (const auto& b : g_blocks) held += b.second.n;
+    for (const Pool* q : g_pools) held += q->kept;
+    const size_t reused = pool && pool->kept >= n ? n : 0;
+    if (n > g_limit || held - reused + n > g_capacity) return cudaErrorMemoryAllocation;
     *p = std::calloc(1, n ? n : 1);
     g_blocks[*p] = {n, pool};
     if (pool) pool->kept -= pool->kept < n ? pool->kept : n;
@@ -88,11 +92,18 @@ extern "C" {
 
 // what a test sets and asks
 void fake_limit(size_t bytes) { g_limit = bytes; }           // larger device allocations fail
+void fake_capacity(size_t bytes) { g_capacity = bytes; }     // of the device, what pools keep included
 void fake_refuse_launch(int n) { g_launches_to_error = n; }   // the n-th from here on (0: the next)
 void fake_max_cluster(int ctas) { g_max_cluster = ctas; }     // larger clusters cannot be placed
+void fake_wait(void) { drain_all(); }                         // for the device
 size_t fake_kept(void) {                                      // bytes that pools keep unused
     size_t n = 0;
     for (Pool* p : g_pools) n += p->kept;
+    return n;
+}
+size_t fake_held(void) {  // bytes of live allocations
+    size_t n = 0;
+    for (const auto& b : g_blocks) n += b.second.n;
     return n;
 }
 size_t fake_pending(const void* p, size_t n) {  // queued copies from or to [p, p + n)

@@ -35,7 +35,8 @@ def host(tmp_path_factory):
     mod = _module("spin_glass_b200_host", PKG / "__init__.py")
     mod.LIB_PATH = so
     L = mod.lib()
-    for name, args, res in (("fake_limit", [C.c_size_t], None), ("fake_max_cluster", [C.c_int], None),
+    for name, args, res in (("fake_limit", [C.c_size_t], None), ("fake_capacity", [C.c_size_t], None),
+                            ("fake_held", [], C.c_size_t), ("fake_wait", [], None), ("fake_max_cluster", [C.c_int], None),
                             ("fake_refuse_launch", [C.c_int], None),
                             ("fake_kept", [], C.c_size_t), ("fake_pending", [C.c_void_p, C.c_size_t], C.c_size_t)):
         f = getattr(L, name)
@@ -48,6 +49,7 @@ def fake(host):
     L = host.lib()
     yield L
     L.fake_limit(C.c_size_t(-1).value)
+    L.fake_capacity(C.c_size_t(-1).value)
     L.fake_max_cluster(16)
     L.fake_refuse_launch(-1)
 
@@ -82,3 +84,33 @@ def test_checkpoint_calls_that_fail_are_done_with_the_callers_memory(host, fake,
             else:
                 host._check(fake.csg_save_checkpoint(e._h, host._p(ref), ref.size))
         assert fake.fake_pending(ref.ctypes.data, ref.nbytes) == 0
+
+
+def _stream_call(host, fake):
+    """One call of the streaming engine on a caller's buffers, waited for; the bytes kept after it."""
+    L = 26
+    cfg, _keep = host.make_config(L, 1, 2, BETAS, seed=1)
+    spins = np.zeros(2 * BETAS.size * L ** 3, np.uint32)
+    bonds = np.zeros(3 * L ** 3, np.uint32)
+    host.run_device(cfg, spins.ctypes.data, bonds.ctypes.data, None, 0, 2)
+    fake.fake_wait()
+    return fake.fake_kept()
+
+
+def test_kept_scratch_is_given_back(host, fake):
+    assert _stream_call(host, fake) > 0  # kept for the next call ...
+    host.trim_scratch()                  # ... until the caller wants it
+    assert fake.fake_kept() == 0
+    for make in (lambda: host.Engine(4, 1, 2, BETAS, seed=1), lambda: host.Server(1 << 30, 2, 16),
+                 lambda: host.Batch([dict(L=4, n_words=1, n_copies=2, betas=BETAS, seed=1)])):
+        owner = make()
+        assert _stream_call(host, fake) > 0
+        owner.close()
+        assert fake.fake_kept() == 0
+
+
+def test_kept_scratch_does_not_stand_in_an_engines_way(host, fake):
+    kept = _stream_call(host, fake)
+    fake.fake_capacity(fake.fake_held() + kept + 1000)
+    with host.Engine(4, 1, 1, BETAS, seed=1) as e:
+        e.init_lattice()
