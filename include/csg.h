@@ -185,7 +185,10 @@ int csg_obs_records(csg_engine* e, float* rec, size_t n_floats);
  * site (z*L+y)*L+x, bits 0..T-1 spins by temperature, bits 26..31 the six
  * bonds (-x,+x,-y,+y,-z,+z; bit 1 = ferromagnetic).  Requires
  * n_copies == 2 and n_temps <= 24.  load_checkpoint checks that the bond
- * bits agree between the ends of every bond and between the two copies. */
+ * bits agree between the ends of every bond and between the two copies.
+ * Both calls convert on the device, with scratch for as many sample words
+ * (256 L^3 bytes each) as fit in 256 MiB, at least one; for fewer where the device
+ * has no room, and for one in page-locked host memory where it has none. */
 int csg_save_checkpoint(csg_engine* e, uint32_t* ref, size_t n_words);
 int csg_load_checkpoint(csg_engine* e, const uint32_t* ref, size_t n_words, int64_t sweep);
 

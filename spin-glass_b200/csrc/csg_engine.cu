@@ -1007,7 +1007,7 @@ int csg_detail::engine_create_pooled(const csg_config* cfg, cudaMemPool_t pool, 
     alloc(&e->hist, e->n_hist);
     alloc(&e->swap_acc, (size_t)d.n_copies * d.n_temps);
     alloc(&e->swap_log, (size_t)cfg->swap_log_rounds * e->n_e / 32);
-    alloc(&e->boundary, 1);
+    alloc(&e->boundary, 2);
     if (rc == CSG_OK) rc = reset_obs(e);
     if (rc == CSG_OK) {
         // A launch plan must exist before the engine is handed out.
@@ -1209,23 +1209,40 @@ int csg_set_plan_override(const csg_plan* plan) {
 // ---------------------------------------------------------------------------
 namespace {
 
-// Device scratch of a call, in the order of the engine's stream.
+// Scratch of a call: device memory in the order of the engine's stream, or
+// page-locked host memory, which kernels reach at the same address.
 struct Scratch {
     void* p = nullptr;
+    bool host = false;
     cudaStream_t st;
     explicit Scratch(cudaStream_t s) : st(s) {}
     Scratch(const Scratch&) = delete;
     Scratch& operator=(const Scratch&) = delete;
     ~Scratch() {
-        if (p) cudaFreeAsync(p, st);
+        if (p && host) {
+            cudaStreamSynchronize(st);
+            cudaFreeHost(p);
+        } else if (p) {
+            cudaFreeAsync(p, st);
+        }
     }
-    int take(const csg_engine* e, size_t bytes) {
+    cudaError_t take(const csg_engine* e, size_t bytes) {
         const cudaError_t ce = e->pool ? cudaMallocFromPoolAsync(&p, bytes, e->pool, st)
                                        : scratch_alloc(&p, bytes, st);
-        if (ce == cudaSuccess) return CSG_OK;
-        cudaGetLastError();
-        p = nullptr;
-        return fail(CSG_ERR_NOMEM, std::string("checkpoint scratch: ") + cudaGetErrorString(ce));
+        if (ce != cudaSuccess) {
+            cudaGetLastError();
+            p = nullptr;
+        }
+        return ce;
+    }
+    cudaError_t take_host(size_t bytes) {
+        const cudaError_t ce = cudaHostAlloc(&p, bytes, cudaHostAllocDefault);
+        if (ce != cudaSuccess) {
+            cudaGetLastError();
+            p = nullptr;
+        }
+        host = ce == cudaSuccess;
+        return ce;
     }
 };
 
@@ -1233,17 +1250,23 @@ int checkpoint_failed(cudaError_t ce) {
     return fail(CSG_ERR_CUDA, std::string("checkpoint: ") + cudaGetErrorString(ce));
 }
 
-// Scratch for the checkpoint of `words` words of samples at once (and extra
-// bytes): all of them up to 256 MB, fewer where the device cannot hold that.
+// Scratch for the checkpoint of `words` words of samples at once: all of them
+// up to 256 MiB, fewer where the device cannot hold that, and one word in host
+// memory (the kernels are then bound by the bus, as the copies are otherwise)
+// where it cannot hold one.
 constexpr size_t kCheckpointScratch = (size_t)256 << 20;
-int checkpoint_scratch(const csg_engine* e, Scratch& sc, int& words, size_t extra) {
+int checkpoint_scratch(const csg_engine* e, Scratch& sc, int& words) {
     const csg_dims& d = e->cfg.dims;
     const size_t word = (size_t)64 * d.L * d.L * d.L * 4;
     words = (int)std::max<size_t>(1, std::min<size_t>(std::min(d.n_words, 32767), kCheckpointScratch / word));
-    for (;; words = (words + 1) / 2) {
-        const int rc = sc.take(e, words * word + extra);
-        if (rc == CSG_OK || words == 1) return rc;
+    cudaError_t ce = sc.take(e, words * word);
+    while (ce != cudaSuccess && words > 1) {
+        words = (words + 1) / 2;
+        ce = sc.take(e, words * word);
     }
+    if (ce != cudaSuccess) ce = sc.take_host(word);
+    if (ce == cudaSuccess) return CSG_OK;
+    return fail(CSG_ERR_NOMEM, std::string("checkpoint scratch: ") + cudaGetErrorString(ce));
 }
 
 }  // namespace
@@ -1300,7 +1323,7 @@ int csg_save_checkpoint(csg_engine* e, uint32_t* ref, size_t n_words) {
     if (n_words != (size_t)64 * W * N) return fail(CSG_ERR_ARG, "checkpoint size mismatch");
     int step = 0;
     Scratch sc(e->stream);
-    if (int rc = checkpoint_scratch(e, sc, step, 0)) return rc;
+    if (int rc = checkpoint_scratch(e, sc, step)) return rc;
     uint32_t* dev = static_cast<uint32_t*>(sc.p);
     cudaError_t ce = cudaSuccess;
     for (int w0 = 0; w0 < W && ce == cudaSuccess; w0 += step) {
@@ -1309,8 +1332,8 @@ int csg_save_checkpoint(csg_engine* e, uint32_t* ref, size_t n_words) {
             e->spins, e->bonds, csg::CheckpointDims{L, T, w0, n}, dev);
         ce = cudaGetLastError();
         if (ce == cudaSuccess)
-            ce = cudaMemcpyAsync(ref + (size_t)64 * w0 * N, dev, (size_t)64 * n * N * 4, cudaMemcpyDeviceToHost,
-                                 e->stream);
+            ce = cudaMemcpyAsync(ref + (size_t)64 * w0 * N, dev, (size_t)64 * n * N * 4,
+                                 sc.host ? cudaMemcpyHostToHost : cudaMemcpyDeviceToHost, e->stream);
     }
     // ref is the caller's again when this returns, with an error too
     const cudaError_t done = cudaStreamSynchronize(e->stream);
@@ -1328,14 +1351,13 @@ int csg_load_checkpoint(csg_engine* e, const uint32_t* ref, size_t n_words, int6
     if (n_words != (size_t)64 * W * N) return fail(CSG_ERR_ARG, "checkpoint size mismatch");
     int step = 0;
     Scratch sc(e->stream);
-    if (int rc = checkpoint_scratch(e, sc, step, 8)) return rc;
-    const size_t ref_bytes = (size_t)64 * step * N * 4;
+    if (int rc = checkpoint_scratch(e, sc, step)) return rc;
     uint32_t* dev = static_cast<uint32_t*>(sc.p);
-    auto* first = reinterpret_cast<unsigned long long*>(static_cast<char*>(sc.p) + ref_bytes);
+    auto* first = reinterpret_cast<unsigned long long*>(e->boundary + 1);
     const unsigned nb = (unsigned)((N + 127) / 128);
     auto upload = [&](int w0, int n) {
-        return cudaMemcpyAsync(dev, ref + (size_t)64 * w0 * N, (size_t)64 * n * N * 4, cudaMemcpyHostToDevice,
-                               e->stream);
+        return cudaMemcpyAsync(dev, ref + (size_t)64 * w0 * N, (size_t)64 * n * N * 4,
+                               sc.host ? cudaMemcpyHostToHost : cudaMemcpyHostToDevice, e->stream);
     };
     // check all of it before the engine's state is touched
     unsigned long long bad = 0;

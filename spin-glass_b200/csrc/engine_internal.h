@@ -28,7 +28,7 @@ struct csg_engine {
     int32_t *e_last = nullptr, *m_last = nullptr, *d_last = nullptr;
     uint64_t* swap_acc = nullptr;
     uint32_t* swap_log = nullptr;
-    uint64_t* boundary = nullptr;
+    uint64_t* boundary = nullptr;  // [1]: scratch of csg_load_checkpoint's check
     int64_t sweep = 0, n_meas = 0, swap_rounds = 0, swap_round0 = 0;
     // resident-kernel plan chosen by a batch's tuner or a server (0: automatic)
     int qc = 0;    // quads per CTA

@@ -33,6 +33,7 @@ struct Block {
 
 std::map<void*, Block> g_blocks;
 std::vector<Stream*> g_streams;
+size_t g_host_blocks = 0;
 std::vector<Pool*> g_pools;
 Stream g_default;
 size_t g_limit = SIZE_MAX, g_capacity = SIZE_MAX;
@@ -101,6 +102,7 @@ size_t fake_kept(void) {                                      // bytes that pool
     for (Pool* p : g_pools) n += p->kept;
     return n;
 }
+size_t fake_host_blocks(void) { return g_host_blocks; }  // live page-locked allocations
 size_t fake_held(void) {  // bytes of live allocations
     size_t n = 0;
     for (const auto& b : g_blocks) n += b.second.n;
@@ -120,6 +122,17 @@ int cudaMalloc(void** p, size_t n) { return take(p, n, nullptr); }
 int cudaFree(void* p) {
     drain_all();
     if (p) release(p);
+    return 0;
+}
+int cudaHostAlloc(void** p, size_t n, unsigned) {
+    *p = std::calloc(1, n);
+    ++g_host_blocks;
+    return 0;
+}
+int cudaFreeHost(void* p) {
+    drain_all();
+    --g_host_blocks;
+    std::free(p);
     return 0;
 }
 int cudaMallocAsync(void** p, size_t n, cudaStream_t) { return take(p, n, nullptr); }

@@ -36,7 +36,8 @@ def host(tmp_path_factory):
     mod.LIB_PATH = so
     L = mod.lib()
     for name, args, res in (("fake_limit", [C.c_size_t], None), ("fake_capacity", [C.c_size_t], None),
-                            ("fake_held", [], C.c_size_t), ("fake_wait", [], None), ("fake_max_cluster", [C.c_int], None),
+                            ("fake_held", [], C.c_size_t), ("fake_host_blocks", [], C.c_size_t),
+                            ("fake_wait", [], None), ("fake_max_cluster", [C.c_int], None),
                             ("fake_refuse_launch", [C.c_int], None),
                             ("fake_kept", [], C.c_size_t), ("fake_pending", [C.c_void_p, C.c_size_t], C.c_size_t)):
         f = getattr(L, name)
@@ -114,3 +115,18 @@ def test_kept_scratch_does_not_stand_in_an_engines_way(host, fake):
     fake.fake_capacity(fake.fake_held() + kept + 1000)
     with host.Engine(4, 1, 1, BETAS, seed=1) as e:
         e.init_lattice()
+
+
+@pytest.mark.parametrize("words", [0, 1, 2])
+def test_checkpoint_calls_on_a_full_device(host, fake, words):
+    # the device holds the scratch of no word, one or two of three
+    L, W = 4, 3
+    ref = np.zeros((64 * W, L ** 3), np.uint32)
+    with host.Engine(L, W, 2, BETAS, seed=1) as e:
+        fake.fake_limit(words * 64 * L ** 3 * 4)
+        e.load_checkpoint(ref, 5)
+        assert fake.fake_pending(ref.ctypes.data, ref.nbytes) == 0
+        host._check(fake.csg_save_checkpoint(e._h, host._p(ref), ref.size))
+        assert fake.fake_pending(ref.ctypes.data, ref.nbytes) == 0
+        assert e.get_state()[2] == 5
+    assert fake.fake_host_blocks() == 0
