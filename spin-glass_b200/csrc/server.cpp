@@ -232,7 +232,14 @@ int csg_server_poll(csg_server* s, int64_t* completed, int32_t max_completed,
         const PlanChoice pc = running > 1 && k < plans.size() ? plans[k] : PlanChoice{};
         r.e->qc = pc.qc;
         r.e->nseg = pc.nseg;
-        if (int rc = csg_run(r.e, n)) {
+        int rc = csg_run(r.e, n);
+        if (rc == CSG_ERR_UNSUPPORTED && pc.qc > 0) {
+            // a tile this device cannot place (a cluster of more CTAs than fit;
+            // refused before anything is launched): the plan taken alone
+            r.e->qc = r.e->nseg = 0;
+            rc = csg_run(r.e, n);
+        }
+        if (rc != CSG_OK) {
             failed(r, rc, last_error());
             continue;
         }

@@ -130,3 +130,19 @@ def test_checkpoint_calls_on_a_full_device(host, fake, words):
         assert fake.fake_pending(ref.ctypes.data, ref.nbytes) == 0
         assert e.get_state()[2] == 5
     assert fake.fake_host_blocks() == 0
+
+
+@pytest.mark.parametrize("most", [4, 8, 16])  # ascending: plans that were placed are kept
+def test_requests_whose_tile_cannot_be_placed_take_the_automatic_plan(host, fake, most):
+    # two small requests that share the GPU are given one quad per CTA, clusters of 12
+    # and 8, whatever clusters the device can place
+    fake.fake_max_cluster(most)
+    with host.Server(1 << 30, 4, 16) as srv:
+        ids = [srv.submit(20, L=16, n_words=1, n_copies=2, betas=np.linspace(2.0, 0.5, 24), seed=1),
+               srv.submit(20, L=12, n_words=1, n_copies=2, betas=np.linspace(2.0, 0.5, 16), seed=2)]
+        got = set()
+        for _ in range(10):
+            got |= set(srv.poll()[0])
+        assert got == set(ids)
+        for i in ids:
+            srv.result(i)
