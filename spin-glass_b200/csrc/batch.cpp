@@ -341,6 +341,13 @@ int csg_batch_tune(csg_batch* b, int64_t probe_sweeps, int32_t* chosen) {
     size_t combos = 1;
     for (size_t i = 0; i < n; ++i) {
         options[i] = plan_options(b->eng[i]->cfg, true);
+        // the plan it starts from too: where the GPU is not full the planner picks
+        // larger teams than the tuned splits have
+        const PlanChoice start{b->eng[i]->qc, b->eng[i]->nseg};
+        const bool known = std::any_of(options[i].begin(), options[i].end(), [&](const PlanChoice& o) {
+            return o.qc == start.qc && o.nseg == start.nseg;
+        });
+        if (!known) options[i].push_back(start);
         combos *= std::max<size_t>(1, options[i].size());
     }
     auto set_choice = [&](size_t i, const PlanChoice& pc) {
