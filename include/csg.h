@@ -126,6 +126,8 @@ typedef struct csg_device_obs {
 
 /* Launch plan: quads per CTA, CTAs per sample word (cluster size), threads
  * per quad, dynamic shared memory bytes. */
+/* Launch plan.  The streaming engine without CSG_STREAM_FUSED has no tile: 0, 0, 256
+ * (threads of a block of its passes over the whole state), 0. */
 typedef struct csg_plan {
     int32_t quads_per_cta;
     int32_t ctas_per_word;

@@ -338,7 +338,7 @@ int make_plan(const csg_config& cfg, int field, Plan& out, PlanChoice forced = P
             out.threads = nt;
             out.smem = (size_t)smem;
         } else {  // colour launches
-            out.TPQ = csg::kStreamThreads;
+            out.TPQ = csg::kStreamThreads;  // the passes over the whole state (colour launches run 128)
         }
         return CSG_OK;
     }

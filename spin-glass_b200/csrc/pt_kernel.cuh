@@ -23,10 +23,11 @@ namespace cgx = cooperative_groups;
 
 constexpr int kMaxT = 64;
 constexpr int kMaxThreads = 512;  // CTA size cap: keeps 128 registers per thread available
-// The general-field kernels whose threads each walk a whole column (one
-// segment) keep more state live per site than 128 registers hold (they spilled
-// up to 316 bytes at L = 24); their CTAs are capped at 384 threads, which
-// leaves 168 registers per thread.
+// The field kernels whose threads each walk a whole column (one segment) keep
+// more state live per site than 128 registers hold; their CTAs are capped at 384
+// threads, which leaves 168 registers per thread.  The rule of fields below 2
+// then spills nothing at L = 16 (up to 60 bytes of stores and 80 of loads elsewhere,
+// L = 20), the general rule 60 to 116 and 96 to 152 (pt_resident.cuh, kSiteGroup).
 constexpr int kMaxThreadsGenWalk = 384;
 __host__ __device__ constexpr int max_cta_threads(bool gen, int nseg) {
     return gen && nseg == 1 ? kMaxThreadsGenWalk : kMaxThreads;
@@ -383,6 +384,7 @@ __device__ __forceinline__ FlipTerms flip_h0_terms(uint32_t sa, uint32_t ca, uin
     const uint32_t h = lop3<0x7E>(sa, m2, g);
     return FlipTerms{lop3<0xE2>(ca, g, h), lop3<0xD4>(sb, m1, h)};
 }
+// the flip as one word (no kernel takes it: they use flipped below)
 __device__ __forceinline__ uint32_t flip_h0(uint32_t sa, uint32_t ca, uint32_t sb, uint32_t cb,
                                             uint32_t r, uint32_t t0, uint32_t t1, uint32_t t2) {
     const FlipTerms f = flip_h0_terms(sa, ca, sb, cb, r, t0, t1, t2);

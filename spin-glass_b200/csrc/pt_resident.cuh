@@ -75,6 +75,11 @@ constexpr int kUnrollAllZS = CSG_UNROLL_ALL_ZS;
 // pass, ~750 bytes a site, then fall out of the instruction cache.  Groups
 // that do not tile the column, with a shorter tail, were slower too (L = 14,
 // 10 words: 7.4 against 6.5 us with groups of 2).
+// The general rule (H >= 2) spills more in groups of 8 and 10 than it did in groups
+// of 4 (L = 16: 116 bytes stored, 132 loaded, from none) and is still the
+// faster for this and the other changes: H = 2.5, exchange every 16 sweeps, L =
+// 16 7066 -> 6100 us for 256 sweeps, L = 20 1528 -> 1228 and L = 24 2553 -> 2148
+// for 64.
 constexpr int kSiteGroup = 10;
 
 __host__ __device__ constexpr int site_group(int zs) {
